@@ -355,9 +355,11 @@ SCRS_API int32_t scrs_dec_finalize_into_with_device(scrs_decoder* dec, uint8_t* 
  * encode gives the repairs of k in-order feeds (tower/encoder.rs:89-131), a
  * tower decode the lazy decoder's reconstruction (tower/decoder.rs:218-546).
  * Per-stripe decode matrices are built on the device; GF(256) and tower
- * stripes drain through one persistent kernel per field.  All pointers in a
- * stripe descriptor are device pointers except `indices`, which is host
- * memory read during submit. */
+ * stripes drain through one persistent kernel per field, and where a field's
+ * stripes gain by the tensor cores through another for those (two where only
+ * some of their rows are 16-byte aligned).  All pointers in a stripe descriptor
+ * are device pointers except `indices`, which is host memory read during
+ * submit. */
 enum { SCRS_OP_ENCODE = 0, SCRS_OP_DECODE = 1 };
 
 typedef struct scrs_stripe_desc {
@@ -410,8 +412,8 @@ SCRS_API int32_t scrs_stripe_batch_set_host(scrs_stripe_batch* batch,
                                             const scrs_stripe_desc* descs,
                                             uint64_t count, scrs_error* err);
 /* Run the uploaded stripes on `stream`: one device-side plan kernel builds
- * every decode matrix, one persistent kernel drains the work queue.  With
- * use_graph != 0 the pair is captured once into a CUDA graph and replayed. */
+ * every decode matrix, persistent kernels drain the work queue.  With
+ * use_graph != 0 they are captured once into a CUDA graph and replayed. */
 SCRS_API int32_t scrs_stripe_batch_run(scrs_stripe_batch* batch, void* stream,
                               int32_t use_graph, scrs_error* err);
 /* Baseline form of the same work: one plan launch and one kernel launch per
@@ -421,14 +423,14 @@ SCRS_API int32_t scrs_stripe_batch_run_plain(scrs_stripe_batch* batch, void* str
 /* Number of kernels the last run launched (for launch accounting). */
 SCRS_API uint64_t scrs_stripe_batch_last_launches(const scrs_stripe_batch* batch);
 /* Measurement form of scrs_stripe_batch_run (no graph): brackets the plan
- * launch and the persistent drain launch with CUDA events on `stream`,
- * synchronises, and reports each launch's device time in milliseconds. */
+ * launch and the persistent drain launches with CUDA events on `stream`,
+ * synchronises, and reports their device times in milliseconds. */
 SCRS_API int32_t scrs_stripe_batch_run_timed(scrs_stripe_batch* batch, void* stream,
                                              float* plan_ms, float* drain_ms,
                                              scrs_error* err);
 /* As scrs_stripe_batch_run_timed, with the drain split: the kernels
  * specialised to encode matrices (spec_ms, 0 when there are none) and the
- * generic drain (generic_ms); drain_ms above is their sum. */
+ * others (generic_ms); drain_ms above is their sum. */
 SCRS_API int32_t scrs_stripe_batch_run_timed_drains(scrs_stripe_batch* batch, void* stream,
                                                     float* plan_ms, float* spec_ms,
                                                     float* generic_ms, scrs_error* err);
@@ -437,8 +439,9 @@ SCRS_API int32_t scrs_stripe_batch_run_timed_drains(scrs_stripe_batch* batch, vo
 SCRS_API int32_t scrs_stripe_batch_check(scrs_stripe_batch* batch, scrs_error* err);
 
 /* ---- Autotuner for the persistent drain ----------------------------------
- * No reference counterpart.  Two launch parameters of the drain kernel are
- * tuned per batch geometry:
+ * No reference counterpart.  Two launch parameters of the GF(256) multiply-XOR
+ * drain kernel are tuned per batch geometry (the tensor-core and specialised
+ * drains have none; a batch that runs in those alone keeps the defaults):
  *   seg_rows     input rows staged in shared memory per segment (1..32).
  *                Stripes with more inputs than this pass over their output
  *                rows once per segment; more rows cost shared memory per CTA

@@ -5,8 +5,10 @@
 //   set():  validate descriptors, build per-stripe tasks and the decode
 //           lists on the host, upload everything in one copy;
 //   run():  one plan launch builds every decode matrix on the device (the
-//           closed-form reduced Cauchy solve), one persistent launch drains
-//           the (stripe, chunk) work queue; optionally replayed as a graph;
+//           closed-form reduced Cauchy solve), persistent launches drain the
+//           (stripe, chunk) work queue, one per field and kind of drain
+//           (specialised encodes, XOR networks, tensor cores); optionally
+//           replayed as a graph;
 //   run_plain(): the same work as one plan + one multiply-XOR launch per
 //           stripe, the baseline the persistent form is measured against.
 //
@@ -117,6 +119,15 @@ struct scrs_stripe_batch {
     // Tower stripes (GF((2^8)^2)) take the items [gen_hi, total_items) and
     // their own persistent drain; their plans are plans[plans16_lo, end).
     uint32_t gen_hi = 0, max_in16 = 1, max_plan_r16 = 0, plans16_lo = 0;
+    // Of each field's generic tasks, those that gain by it drain on the tensor
+    // cores (on_tensor_cores): items [lo, hi) at the end of the field's range,
+    // `chunk` row bytes each.  [field][0]: rows of 16-byte units, [1]: the others.
+    struct MxtRun {
+        uint32_t lo = 0, hi = 0, max_in = 1, max_out = 1, chunk = 0;
+        int align = 16;
+        uint64_t blocks = 0;
+    } mxt[2][2];
+    uint32_t alu_hi[2] = {0, 0};  // end of each field's multiply-XOR items
     int shape16 = kShapeAny;
     std::map<std::pair<uint32_t, uint32_t>, std::vector<uint16_t>> tower_coef;  // host tables by (k, m)
     std::vector<uint16_t> l_row_of, l_missing, l_present, l_repairs;  // per-stripe list scratch
@@ -195,6 +206,39 @@ namespace {
 constexpr size_t kMaxPieces = 64;  // one work counter each in d_counter
 constexpr size_t kMaxSpecRuns = 4;  // specialised groups per batch (counters 1..4)
 constexpr size_t kTowerCounter = 1 + kMaxSpecRuns;  // work counter of the tower drain
+constexpr size_t kMxtCounter = kTowerCounter + 1;   // the tensor-core drains': [field][alignment]
+constexpr size_t kRunCounters = kMxtCounter + 4;
+// Most blocks of a tensor-core item: whole rows up to 8 KiB (16 KiB tower).
+constexpr uint32_t kMxtItemBlocks = 32;
+// Fewest blocks per SM that are worth the kernel's set-up (tensor memory,
+// tables, the first operands: several microseconds).
+constexpr uint32_t kMxtMinBlocksPerSm = 8;
+
+// Largest of 16, 8 and 1 that every row of T is aligned to.
+int row_align(const MxkTask& T) {
+    const uint64_t low = T.L | reinterpret_cast<uintptr_t>(T.in) | reinterpret_cast<uintptr_t>(T.out);
+    return low % 16 == 0 ? 16 : low % 8 == 0 ? 8 : 1;
+}
+
+// Whether task T of a device-resident batch drains on the tensor cores
+// (mxt_kernels.cu).  Their time follows the input bytes, the XOR networks'
+// inputs times outputs, so the line lies at a product; below 16 or 24 inputs a
+// K = 64 step is mostly padding.  Rows that are not in 16-byte units cost the
+// XOR networks byte accesses, the tensor cores little.  Measured as time of the
+// XOR networks over time of the tensor cores, batches of 160 MB, 4096-byte rows:
+//   GF(256), k x m:  16 x 16  0.86   24 x 12 1.03   32 x 6 1.07   32 x 8 1.15
+//                    64 x 3  1.16    64 x 16 3.1    128 x 16 3.2   32 x 20 (two passes) 1.11
+//   tower:           8 x 4  0.78     16 x 2 1.08    32 x 1 1.29   32 x 8 3.2   64 x 8 4.5
+// and with 1400-byte rows:
+//   GF(256):         16 x 4 0.92     16 x 5 1.06    24 x 2 1.30   32 x 8 2.8   64 x 16 6.8
+//   tower:           8 x 4  0.99     8 x 6 1.22     16 x 1 1.28   32 x 8 3.4
+bool on_tensor_cores(const scrs_stripe_batch* b, const MxkTask& T, int gf16) {
+    if (b->compact_decode || T.n_out == 0 || T.L >> 32 || !mxt_fits(gf16, T.n_in, T.n_out)) return false;
+    const uint32_t product = T.n_in * T.n_out, passes = (T.n_out + (gf16 ? 7 : 15)) / (gf16 ? 8 : 16);
+    if (row_align(T) == 16) return gf16 ? T.n_in >= 16 && product >= 32 : T.n_in >= 24 && product >= 256 * passes;
+    return gf16 ? T.n_in >= 16 || (T.n_in >= 8 && T.n_out >= 6 && passes == 1)
+                : T.n_in >= 24 || (T.n_in >= 16 && T.n_out >= 5);
+}
 
 // g^i for i < 65535 (tower/cauchy.rs:44-49) on the current device: the x and
 // y coordinates every tower decode plan reads.  Uploaded once per device.
@@ -512,30 +556,53 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
     }
     b->gen_lo = next;
     uint32_t max_in = 1, max_in16 = 1;
-    for (int pass = 0; pass < 2; pass++) {
+    for (int f = 0; f < 2; f++) {
+        // the tensor-core tasks of each alignment; too few blocks stay with the
+        // others
+        std::vector<uint8_t> on(count, 0);  // 1 + alignment class
+        bool all_aligned = true, all_whole = true;  // of the others
+        for (int c = 0; c < 2; c++) b->mxt[f][c] = scrs_stripe_batch::MxtRun{};
+        const uint32_t block = mxt_block(f);
         for (uint64_t t = 0; t < count; t++) {
-            if (in_spec[t] || b->task_gf16[t] != pass) continue;
-            b->tasks[t].item_begin = next;
-            next += b->tasks[t].n_items;
-            uint32_t& mx = pass ? max_in16 : max_in;
-            mx = std::max(mx, b->tasks[t].n_in);
+            if (in_spec[t] || b->task_gf16[t] != f || !on_tensor_cores(b, b->tasks[t], f)) continue;
+            const int align = row_align(b->tasks[t]);
+            on[t] = align == 16 ? 1 : 2;
+            scrs_stripe_batch::MxtRun& M = b->mxt[f][on[t] - 1];
+            M.blocks += (b->tasks[t].L + block - 1) / block;
+            M.max_in = std::max(M.max_in, b->tasks[t].n_in);
+            M.max_out = std::max(M.max_out, b->tasks[t].n_out);
+            M.align = std::min(M.align, align);
         }
-        if (pass == 0) b->gen_hi = next;
+        for (int c = 0; c < 3; c++) {
+            if (c) b->mxt[f][c - 1].lo = next;
+            const uint64_t blocks = c ? b->mxt[f][c - 1].blocks : 0;
+            const uint32_t chunk = block * (uint32_t)std::max<uint64_t>(
+                                               1, std::min<uint64_t>(kMxtItemBlocks, blocks / (8ull * b->sm_count)));
+            for (uint64_t t = 0; t < count; t++) {
+                if (in_spec[t] || b->task_gf16[t] != f) continue;
+                if (on[t] && b->mxt[f][on[t] - 1].blocks < (uint64_t)kMxtMinBlocksPerSm * b->sm_count) on[t] = 0;
+                if (on[t] != c) continue;
+                MxkTask& T = b->tasks[t];
+                uint32_t& mx = f ? max_in16 : max_in;
+                mx = std::max(mx, T.n_in);
+                if (c)
+                    T.n_items = (uint32_t)((T.L + chunk - 1) / chunk);
+                else
+                    all_aligned &= T.aligned != 0, all_whole &= T.L % FieldGeom<0>::kChunk == 0;
+                T.item_begin = next;
+                next += T.n_items;
+            }
+            if (c)
+                b->mxt[f][c - 1].hi = next, b->mxt[f][c - 1].chunk = chunk;
+            else
+                b->alu_hi[f] = next;
+        }
+        (f ? b->shape16 : b->shape) = !all_aligned ? kShapeAny : all_whole ? (kShapeAligned | kShapeWhole) : kShapeAligned;
+        if (f == 0) b->gen_hi = next;
     }
     b->total_items = next;
     b->max_in = max_in;
     b->max_in16 = max_in16;
-    auto shape_of = [&](uint8_t gf16) {
-        bool all_aligned = true, all_whole = true;
-        for (size_t t = 0; t < b->tasks.size(); t++) {
-            if (b->task_gf16[t] != gf16) continue;
-            all_aligned &= b->tasks[t].aligned != 0;
-            all_whole &= b->tasks[t].L % FieldGeom<0>::kChunk == 0;
-        }
-        return !all_aligned ? kShapeAny : all_whole ? (kShapeAligned | kShapeWhole) : kShapeAligned;
-    };
-    b->shape = shape_of(0);
-    b->shape16 = shape_of(1);
     b->item_task.resize(next);
     for (size_t t = 0; t < b->tasks.size(); t++)
         std::fill(b->item_task.begin() + b->tasks[t].item_begin,
@@ -773,7 +840,7 @@ DrainCfg drain_cfg(const scrs_stripe_batch* b) {
     }
     const int fit = mxk_ctas_per_sm(c.seg_rows, drain_shape(b, c.seg_rows));
     if (c.ctas_per_sm <= 0 || c.ctas_per_sm > fit) c.ctas_per_sm = fit;
-    const uint32_t items = b->gen_hi - b->gen_lo;
+    const uint32_t items = b->alu_hi[0] - b->gen_lo;
     c.grid = std::max(1, std::min<int>(b->sm_count * c.ctas_per_sm, (int)std::max<uint32_t>(items, 1)));
     return c;
 }
@@ -784,7 +851,7 @@ DrainCfg drain_cfg16(const scrs_stripe_batch* b) {
     DrainCfg c{std::max(1, std::min((int)b->max_in16, FieldGeom<1>::kSegMax)), 0, 0};
     const int shape = b->shape16 | ((int)b->max_in16 <= c.seg_rows ? kShapeOneSeg : 0);
     c.ctas_per_sm = mxk_ctas_per_sm(c.seg_rows, shape, 1);
-    const uint32_t items = b->total_items - b->gen_hi;
+    const uint32_t items = b->alu_hi[1] - b->gen_hi;
     c.grid = std::max(1, std::min<int>(b->sm_count * c.ctas_per_sm, (int)std::max<uint32_t>(items, 1)));
     return c;
 }
@@ -799,19 +866,27 @@ int32_t enqueue_drains(scrs_stripe_batch* b, cudaStream_t st, scrs_error* err, b
                              b->d_counter.as<uint32_t>() + 1 + q, b->status.dev, b->sm_count * R.jk.ctas_per_sm, st));
         b->last_launches++;
     }
-    if (run_generic && b->gen_hi > b->gen_lo) {
+    if (run_generic && b->alu_hi[0] > b->gen_lo) {
         const DrainCfg c = drain_cfg(b);
-        SCRS_CUDA(launch_gf256_mxk(b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), b->gen_lo, b->gen_hi,
+        SCRS_CUDA(launch_gf256_mxk(b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), b->gen_lo, b->alu_hi[0],
                                    b->d_counter.as<uint32_t>(), b->status.dev, c.seg_rows, c.grid, st,
                                    drain_shape(b, c.seg_rows)));
         b->last_launches++;
     }
-    if (run_generic && b->total_items > b->gen_hi) {
+    if (run_generic && b->alu_hi[1] > b->gen_hi) {
         const DrainCfg c = drain_cfg16(b);
         const int shape = b->shape16 | ((int)b->max_in16 <= c.seg_rows ? kShapeOneSeg : 0);
-        SCRS_CUDA(launch_gf256_mxk(b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), b->gen_hi,
-                                   b->total_items, b->d_counter.as<uint32_t>() + kTowerCounter, b->status.dev,
-                                   c.seg_rows, c.grid, st, shape, 1));
+        SCRS_CUDA(launch_gf256_mxk(b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), b->gen_hi, b->alu_hi[1],
+                                   b->d_counter.as<uint32_t>() + kTowerCounter, b->status.dev, c.seg_rows, c.grid, st,
+                                   shape, 1));
+        b->last_launches++;
+    }
+    for (int q = 0; run_generic && q < 4; q++) {
+        const scrs_stripe_batch::MxtRun& M = b->mxt[q >> 1][q & 1];
+        if (M.hi == M.lo) continue;
+        SCRS_CUDA(launch_mxt(b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), M.lo, M.hi,
+                             b->d_counter.as<uint32_t>() + kMxtCounter + q, b->status.dev, M.max_in, M.max_out, M.chunk,
+                             b->sm_count, st, M.align, q >> 1));
         b->last_launches++;
     }
     return SCRS_OK;
@@ -837,7 +912,7 @@ int32_t enqueue_plans(scrs_stripe_batch* b, cudaStream_t st, scrs_error* err) {
 // specialised drains' tails leave idle; the drains touch disjoint items and
 // outputs.  Under graph capture the fork and join become graph edges.
 int32_t enqueue_batch(scrs_stripe_batch* b, cudaStream_t st, scrs_error* err) {
-    SCRS_CUDA(cudaMemsetAsync(b->d_counter.p, 0, (kTowerCounter + 1) * sizeof(uint32_t), st));
+    SCRS_CUDA(cudaMemsetAsync(b->d_counter.p, 0, kRunCounters * sizeof(uint32_t), st));
     b->last_launches = 0;
     const bool fork = !b->spec.empty() && b->total_items > b->gen_lo;
     if (fork) {
@@ -1032,8 +1107,9 @@ extern "C" int32_t scrs_stripe_batch_run_plain(scrs_stripe_batch* b, void* strea
     size_t pi[2] = {0, b->plans16_lo};  // next plan of each field
     const size_t pend[2] = {b->plans16_lo, b->plans.size()};
     for (size_t t = 0; t < b->tasks.size(); t++) {
-        const MxkTask& T = b->tasks[t];
+        MxkTask T = b->tasks[t];
         const int f = b->task_gf16[t];
+        T.n_items = n_chunks(T.L, f != 0);
         // decode stripes carry row lists (encodes none); with erasures they have a plan
         if (T.in_rows && T.n_out && pi[f] < pend[f]) {
             SCRS_CUDA(launch_cauchy_plan_single(b->plans[pi[f]++], f, st));
@@ -1066,7 +1142,7 @@ extern "C" int32_t scrs_stripe_batch_run_timed_drains(scrs_stripe_batch* b, void
     cudaStream_t st = (cudaStream_t)stream;
     cudaEvent_t ev[4];
     for (auto& e : ev) SCRS_CUDA(cudaEventCreate(&e));
-    SCRS_CUDA(cudaMemsetAsync(b->d_counter.p, 0, (kTowerCounter + 1) * sizeof(uint32_t), st));
+    SCRS_CUDA(cudaMemsetAsync(b->d_counter.p, 0, kRunCounters * sizeof(uint32_t), st));
     b->last_launches = 0;
     cudaEventRecord(ev[0], st);
     int32_t rp = enqueue_plans(b, st, err);
@@ -1118,7 +1194,7 @@ int32_t time_drain(scrs_stripe_batch* b, cudaStream_t st, int seg_rows, int grid
     for (uint32_t rep = 0; rep <= reps; rep++) {
         SCRS_CUDA(cudaMemsetAsync(b->d_counter.p, 0, 4, st));
         SCRS_CUDA(cudaEventRecord(e0, st));
-        SCRS_CUDA(launch_gf256_mxk(b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), b->gen_lo, b->gen_hi,
+        SCRS_CUDA(launch_gf256_mxk(b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), b->gen_lo, b->alu_hi[0],
                                    b->d_counter.as<uint32_t>(), b->status.dev, seg_rows, grid, st,
                                    drain_shape(b, seg_rows)));
         SCRS_CUDA(cudaEventRecord(e1, st));
@@ -1140,7 +1216,7 @@ extern "C" int32_t scrs_stripe_batch_autotune(scrs_stripe_batch* b, void* stream
     if (reps > 100) return set_err(err, SCRS_ERR_BAD_ARGUMENT, 3, reps);
     if (reps == 0) reps = 5;
     cudaStream_t st = (cudaStream_t)stream;
-    if (b->gen_hi <= b->gen_lo) return scrs_stripe_batch_launch_params(b, chosen, err);
+    if (b->alu_hi[0] <= b->gen_lo) return scrs_stripe_batch_launch_params(b, chosen, err);
     // inputs on the device and decode matrices built before any drain
     if (b->host_mode) {
         int32_t r = run_host(b, st, err);
@@ -1169,7 +1245,7 @@ extern "C" int32_t scrs_stripe_batch_autotune(scrs_stripe_batch* b, void* stream
             if (std::find(ctas.begin(), ctas.end(), c) == ctas.end()) ctas.push_back(c);
         }
         for (int c : ctas) {
-            const int grid = std::max(1, std::min<int>(b->sm_count * c, (int)(b->gen_hi - b->gen_lo)));
+            const int grid = std::max(1, std::min<int>(b->sm_count * c, (int)(b->alu_hi[0] - b->gen_lo)));
             float ms = 0;
             rc = time_drain(b, st, seg, grid, reps, e0, e1, &ms, err);
             if (rc) break;

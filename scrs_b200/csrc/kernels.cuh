@@ -111,6 +111,17 @@ constexpr int kShapeAny = 0, kShapeAligned = 1, kShapeWhole = 2, kShapeOneSeg = 
 cudaError_t launch_gf256_mxk(const MxkTask* tasks, const uint32_t* item_task, uint32_t item_lo, uint32_t item_end,
                              uint32_t* work_counter, int32_t* status, int seg_rows, int grid, cudaStream_t stream,
                              int shape = kShapeAny, int gf16 = 0);
+// The same drain on the tensor cores (mxt_kernels.cu), for tasks of at most
+// max_in inputs and max_out outputs (mxt_fits).  An item is `chunk` bytes of the
+// rows, a multiple of mxt_block; align (16, 8 or 1): L and every row of every
+// task are multiples of it.
+bool mxt_fits(int gf16, uint32_t max_in, uint32_t max_out);
+uint32_t mxt_block(int gf16);
+cudaError_t launch_mxt(const MxkTask* tasks, const uint32_t* item_task, uint32_t item_lo, uint32_t item_end,
+                       uint32_t* work_counter, int32_t* status, uint32_t max_in, uint32_t max_out, uint32_t chunk,
+                       int grid, cudaStream_t stream, int align, int gf16);
+// Its one-time per-device set-up.
+cudaError_t prepare_mxt();
 // One task by value; grid <= 0 means one CTA per row chunk (or the
 // input-split form for more than one segment of inputs, see below).  `chain`:
 // the input-split form's launches use programmatic dependent launch, so they

@@ -776,6 +776,7 @@ cudaError_t prepare_batch_kernels() {
     cudaError_t e = ensure_tables();
     if (e == cudaSuccess) e = set_mxk_attrs<0>();
     if (e == cudaSuccess) e = set_mxk_attrs<1>();
+    if (e == cudaSuccess) e = prepare_mxt();
     return e;
 }
 
