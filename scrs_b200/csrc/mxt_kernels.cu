@@ -26,29 +26,37 @@
 // operations per input word for four operand words, against the XOR
 // networks' work per (input, output) pair.
 //
-// One persistent CTA per SM, 20 warps: a publisher (claims work items), the MMA
-// issuer, two builders of B, two epilogue groups of four warps (counts -> parities
-// -> bytes -> rows, one per tile) and two expander groups of four warps (rows -> A,
-// alternate units; they also write decode's present rows through).  A block is 256
-// columns, two tiles of 128: a thread expands one column of each, and its results
-// stay in its own tensor-memory lane.  A flows through a ring of units and D
-// through a ring of tiles, so loads, expansion, MMAs and epilogue overlap.
+// One persistent CTA per SM, 25 warps: a publisher (claims work items), two MMA
+// issuers (one for each tile of a block), two builders of B, two epilogue groups of
+// four warps (counts -> parities -> bytes -> rows, alternate blocks), two expander
+// groups of four warps (staged rows -> A, alternate units; they also write decode's
+// present rows through) and four loaders (rows -> shared memory).  A block is 256
+// columns, two tiles of 128: a thread holds two neighbouring columns, one of each
+// tile, so it reads and writes both at once, and its results stay in its own
+// tensor-memory lane.  Rows flow through a ring of staged units, A through a ring
+// of units and D through a ring of tiles, so loads, expansion, MMAs and epilogue
+// overlap.
 //
-// What bounds it: no pipe does.  At 64 inputs and 16 outputs a block of 256
-// columns takes 2660 cycles: 1024 of MMAs and 1460 of issue slots (5820
-// instructions, nearly half of them on the ALU pipe); the rest is latency between
-// the roles, whose chain of hand-overs the A ring (three units) and the
-// accumulator ring (one or two blocks) only partly hide.
-// Measured against the XOR networks (drain alone, half encodes, half decodes of
-// random losses): GF(256) 64 + 16, 4096-byte rows 700 -> 324 us for 872 MB of
-// rows; 32 + 8, 1400-byte rows 1123 -> 386 us for 596 MB; tower 32 + 8, 64 KiB rows
-// 821 -> 290 us for 872 MB.
+// What bounds it: no pipe alone.  At 64 inputs and 16 outputs a block takes about
+// 1900 cycles, of which the tensor pipe works 52 % (1150 are the least for 18 MMAs),
+// the ALU pipe 54 %, shared memory 56 % and the issue slots 59 % (4900
+// instructions); the rest is latency between the roles.
+// Drains by CUDA events, whole batches with their plan, half encodes and half decodes
+// of random losses: GF(256) 64 + 16, 4096-byte rows 278 us for 872 MB of rows
+// (346 with one issuer, loads in the expanders and 128 separate columns a tile); 32 +
+// 8, 1400-byte rows 238 us for 596 MB (389); tower 32 + 8, 64 KiB rows 282 us
+// for 872 MB (319).
 //
-// Choices, with what the alternatives took (the 64 + 16 batch): units of two
-// steps 424 us and of three 404 against 377 with four; three expander groups 415
-// against 400 with two; polls with a time hint 401 against 384 without; A in
-// shared memory and the columns on the N side, whose epilogue needs no staging,
-// 437 against 401.
+// Choices, with what the alternatives took.  A lane's two columns neighbours instead
+// of 128 apart, and staging of one's own warp instead of the group's in the
+// epilogue: 346 -> 286 us (64 + 16).  Loader warps instead of copies issued by the
+// expanders: 356 -> 273 us (1400-byte rows).  An issuer per tile, and epilogue groups
+// that alternate blocks instead of sharing each: 274 -> 244 us (1400), 286 -> 276
+// (64 + 16), 363 -> 331 (32 + 8 of 4096 bytes).  Eight staged units instead of six:
+// 244 -> 238 us (1400).  Sleeps between the polls of the roles that are ahead: no
+// difference.  Of the first form (377 us for 64 + 16): units of two steps 424, of
+// three 404, against four; polls with a time hint 401 against 384 without; A in
+// shared memory and the columns on the N side 437 against 401.
 
 #include <algorithm>
 #include <atomic>
@@ -62,7 +70,9 @@ namespace scrs {
 namespace {
 
 constexpr int kEpiWarp = 4, kExpWarp = 12, kExpGroups = 2;
-constexpr int kMxtThreads = 32 * (kExpWarp + 4 * kExpGroups);
+constexpr int kLoadWarp = kExpWarp + 4 * kExpGroups;
+constexpr int kMma1Warp = kLoadWarp + 4;  // the second tile's issuer; the first tile's is warp 1
+constexpr int kMxtThreads = 32 * (kMma1Warp + 1);
 constexpr uint32_t kStepCols = 16;                    // tensor-memory columns of a step's A operand (two tiles)
 constexpr uint32_t kUnitSteps = 4;                    // K = 64 steps handed over at once (a block's last unit may hold fewer)
 constexpr uint32_t kUnitCols = kUnitSteps * kStepCols;
@@ -73,16 +83,18 @@ constexpr uint32_t kScaleCol = 496;                   // tensor-memory columns o
 // bit 12 is the parity.
 constexpr uint32_t kSixes = 0x77777777u;              // eight elements of 6
 constexpr uint32_t kBiasCol = 488;                    // tensor-memory columns of the constant A operand
-constexpr uint32_t kDepth = 2;       // units an expander warp has loaded or in flight
-constexpr uint32_t kStage = 784;     // staged bytes of a step's rows, 2 x 32 columns' worth, and 16 for their leads
-constexpr uint32_t kUnit = kUnitSteps * kStage;
-constexpr uint32_t kAhead = (kDepth + 1) * kExpGroups;  // the loads' lead over the last warp's work, in units
+constexpr uint32_t kStages = 8;      // units of rows loaded or in flight
+constexpr uint32_t kUnit = 32 * 320 + 32;  // a unit's staged rows (32 of 320 or 16 of 528), their leads
+constexpr uint32_t kLeads = kUnit - 32;
+constexpr uint32_t kEpiStage = 64 * kGroupBytes + 16;  // an epilogue warp's staging: 64 columns, and a word past them
+constexpr uint32_t kAhead = kStages + 6;  // the loads' lead over the last warp's work, in units
 constexpr uint32_t kItemSlots = kAhead + 4;
 constexpr uint32_t kBiasBytes = 128 * 32;  // the constant B operand
 constexpr uint32_t kMaxRows = 256;
 constexpr uint32_t kMaxBytes = 223;  // input field bytes of a task: at most 1791 counts
 constexpr uint8_t kNoPass = 255;      // no output row (data rows end at 254)
 constexpr uint32_t kMaxRing = 16;
+constexpr uint32_t kDBars = 4;  // accumulator tiles' barriers: two blocks', one for each epilogue group
 
 // A work item as the roles read it: rows [in + row[i] * in_stride, + len).
 struct ItemSlot {
@@ -91,7 +103,7 @@ struct ItemSlot {
     const void* coef;
     const uint16_t* coef_rows;
     uint32_t in_stride, out_stride;
-    uint32_t len, rest;        // bytes of the item; bytes to the end of the rows
+    uint32_t len, rest;        // bytes of the item; and to the end of the rows, up to 16 bytes past the item's
     uint32_t n_in, n_out, ld;
     uint32_t steps, units, passes, per, blocks;
     uint32_t valid, accumulate, copies;
@@ -101,12 +113,12 @@ struct ItemSlot {
 };
 
 struct Bars {
+    uint64_t raw_full[kStages], raw_empty[kStages];
     uint64_t exp_full[kMaxRing], exp_empty[kMaxRing];
-    uint64_t d_full[kMaxRing], d_empty[kMaxRing];
+    uint64_t d_full[kDBars], d_empty[kDBars];
     uint64_t b_full[2], b_empty[2];
-    uint64_t stg_full[2], stg_empty[2];
     uint64_t item_full[kItemSlots], item_empty[kItemSlots];
-    uint64_t fin;
+    uint64_t fin[2];
     uint32_t tmem, abort;
 };
 
@@ -221,6 +233,22 @@ __device__ __forceinline__ void mma_step(uint32_t d, uint32_t a, uint64_t b, uin
         "r"(a), "l"(b), "r"(idesc), "r"(scale), "n"(kAccumulate ? 1 : 0)
         : "memory");
 }
+// A whole unit's steps, n2 descriptor units of B apart, then the arrival at
+// `bar` when they end: one election, and one conversion of the common operands.
+__device__ __forceinline__ void mma_unit(uint32_t d, uint32_t a, uint64_t b, uint32_t n2, uint32_t idesc, uint32_t scale,
+                                         uint64_t* bar) {
+    static_assert(kUnitSteps == 4, "four MMAs below");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], %5, %9, [%10], [%10], 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%2], %6, %9, [%10], [%10], 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%3], %7, %9, [%10], [%10], 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%4], %8, %9, [%10], [%10], 1;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%11];\n\t}" ::"r"(d),
+        "r"(a), "r"(a + kStepCols), "r"(a + 2 * kStepCols), "r"(a + 3 * kStepCols), "l"(b), "l"(b + n2), "l"(b + 2 * n2),
+        "l"(b + 3 * n2), "r"(idesc), "r"(scale), "r"(smem_addr(bar))
+        : "memory");
+}
 __device__ __forceinline__ void tmem_store8(uint32_t addr, const uint4& a, const uint4& b) {  // this lane's 8 columns
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(a.x),
                  "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
@@ -251,8 +279,10 @@ template <int kGf16>
 struct MxtGeom {
     static constexpr uint32_t kElem = kGf16 ? 2 : 1;         // field bytes of a symbol element
     static constexpr uint32_t kRow = 256 * kElem;            // bytes of a row per block
-    static constexpr uint32_t kTile = 128 * kElem;           // and per tile
-    static constexpr uint32_t kSpan = 32 * kElem;            // of which an expander warp's lanes hold
+    // and per staged row: with a piece for its lead, and two of a GF(256) unit's
+    // rows in different banks
+    static constexpr uint32_t kPitch = kRow + (kGf16 ? 16 : 64);
+    static constexpr uint32_t kSpan = 64 * kElem;            // of which a warp's lanes hold, two columns each
     static constexpr uint32_t kChunkRows = 4 / kElem;        // input rows of a chunk of 4 field bytes
     static constexpr uint32_t kStepRows = 2 * kChunkRows;    // and of a K = 64 step
     static constexpr uint32_t kGroup = kGroupBytes / kElem;  // output rows per pass
@@ -307,11 +337,11 @@ __device__ __forceinline__ void copy_in(uint32_t dst, const void* src, bool on) 
             "l"(src), "r"((uint32_t)on)
             : "memory");
 }
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int kPending>
-__device__ __forceinline__ void copy_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+// This thread's arrival as the copies that it has issued land.
+__device__ __forceinline__ void copy_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
+__device__ __forceinline__ void copy_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---- the kernel ----------------------------------------------------------------
 // kAlign (16, 8 or 1): every row, in and out, starts at a multiple of it and L is
@@ -330,23 +360,21 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
     uint8_t* s_bias = smem + up(sizeof(Head), 128);
     uint8_t* s_b = s_bias + kBiasBytes;
     uint8_t* s_raw = s_b + P.n_b * P.b_bytes;
-    uint8_t* s_stg = s_raw + 4 * kExpGroups * kDepth * kUnit;
+    uint8_t* s_stg = s_raw + kStages * kUnit;
     const int tid = threadIdx.x, lane = tid & 31, warp = (int)uni(tid >> 5);
 
     // ---- set-up: barriers, tables, tensor memory
     if (tid == 0) {
-        for (uint32_t i = 0; i < kMaxRing; i++) {
-            mbar_init(&B->exp_full[i], 4), mbar_init(&B->exp_empty[i], 1);
-            mbar_init(&B->d_full[i], 1), mbar_init(&B->d_empty[i], 4);
-        }
-        for (int i = 0; i < 2; i++) {
-            mbar_init(&B->b_full[i], 2), mbar_init(&B->b_empty[i], 1);
-            mbar_init(&B->stg_full[i], 4), mbar_init(&B->stg_empty[i], 4);
-        }
-        // consumers: MMA issuer, 2 builders, 8 epilogue warps, the expanders
+        for (uint32_t i = 0; i < kMaxRing; i++) mbar_init(&B->exp_full[i], 4), mbar_init(&B->exp_empty[i], 2);
+        for (uint32_t i = 0; i < kDBars; i++) mbar_init(&B->d_full[i], 1), mbar_init(&B->d_empty[i], 4);
+        // a loader thread's arrival as its copies land; a loader warp's for the leads
+        for (uint32_t i = 0; i < kStages; i++)
+            mbar_init(&B->raw_full[i], kAligned ? 128 : 132), mbar_init(&B->raw_empty[i], 4);
+        for (int i = 0; i < 2; i++) mbar_init(&B->b_full[i], 2), mbar_init(&B->b_empty[i], 2);
+        // consumers: 2 MMA issuers, 2 builders, 8 epilogue warps, the expanders, 4 loaders
         for (uint32_t i = 0; i < kItemSlots; i++)
-            mbar_init(&B->item_full[i], 1), mbar_init(&B->item_empty[i], 11 + 4 * kExpGroups);
-        mbar_init(&B->fin, 1);
+            mbar_init(&B->item_full[i], 1), mbar_init(&B->item_empty[i], 16 + 4 * kExpGroups);
+        mbar_init(&B->fin[0], 1), mbar_init(&B->fin[1], 1);
         B->abort = 0;
         fence_mbar_init();
     }
@@ -434,7 +462,8 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                     I.coef_rows = T.coef_rows;
                     I.in_stride = (uint32_t)T.in_stride;
                     I.out_stride = (uint32_t)T.out_stride;
-                    I.rest = (uint32_t)(T.L - off);
+                    const uint64_t rest = T.L - off;
+                    I.rest = (uint32_t)(rest < P.chunk + 16 ? rest : P.chunk + 16);
                     I.len = umin32(I.rest, P.chunk);
                     I.n_in = T.n_in, I.n_out = T.n_out, I.ld = T.ld;
                     I.steps = steps;
@@ -454,88 +483,51 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
             if (!valid) break;
             it.next(kItemSlots);
         }
-    } else if (warp == 1) {
-        // ---- MMA issuer
-        Ring bs, ds, as;
+    } else if (warp == 1 || warp == kMma1Warp) {
+        // ---- MMA issuers, one for each tile of a block
+        const uint32_t tile = warp == 1 ? 0u : 1u;
+        // ds: this tile's barriers; es: those of the tile that last held its
+        // accumulator, n_d tiles before
+        Ring bs, ds, es, as;
+        ds.i = tile, es.i = tile + kDBars - P.n_d;
         const uint64_t bias = operand_desc(smem_addr(s_bias));
         for (;;) {
             warp_wait(&B->item_full[it.i], it.ph, B, P.status);
             const ItemSlot& I = H.item[it.i];
             if (!uni(I.valid) || aborted(B)) break;
-            const uint32_t passes = uni(I.passes), blocks = uni(I.blocks), steps = uni(I.steps), units = uni(I.units),
-                           per = uni(I.per), n_out = uni(I.n_out);
+            const uint32_t passes = uni(I.passes), blocks = uni(I.blocks), steps = uni(I.steps), per = uni(I.per),
+                           n_out = uni(I.n_out);
             for (uint32_t pass = 0; pass < passes; pass++) {
                 const uint32_t N = columns_of<kGf16>(umin32(per, n_out - pass * per));
                 const uint32_t idesc = instr_desc(N), N2 = N * 2;  // N * 32 bytes of B a step
                 warp_wait(&B->b_full[bs.i], bs.ph, B, P.status);
                 const uint64_t b0 = operand_desc(smem_addr(s_b + bs.i * P.b_bytes));
                 for (uint32_t b = 0; b < blocks; b++) {
-                    // one tile after the other where the A ring holds a block's units
-                    // (a tile's epilogue runs beside the other's MMAs), else both at
-                    // every step
-                    if (units <= P.ring) {
-                        const Ring as0 = as;
-#pragma unroll
-                        for (uint32_t tile = 0; tile < 2; tile++) {
-                            warp_wait(&B->d_empty[ds.i], ds.ph ^ 1u, B, P.status);
-                            const uint32_t d = tmem + ds.i * P.d_cols;
-                            tc_fence_after();
-                            mma_step<false>(d, tmem + kBiasCol, bias, idesc, tmem + kScaleCol);
-                            as = as0;
-                            uint64_t bd = b0;
-                            uint32_t left = steps;
-                            for (uint32_t u = 0; u < units; u++) {
-                                if (tile == 0) {
-                                    warp_wait(&B->exp_full[as.i], as.ph, B, P.status);
-                                    tc_fence_after();
-                                }
-                                const uint32_t a = tmem + a_col + as.i * kUnitCols + tile * (kStepCols / 2);
-                                if (left >= kUnitSteps) {
-#pragma unroll
-                                    for (uint32_t h = 0; h < kUnitSteps; h++)
-                                        mma_step<true>(d, a + h * kStepCols, bd + h * N2, idesc, tmem + kScaleCol);
-                                } else {
-#pragma unroll
-                                    for (uint32_t h = 0; h < kUnitSteps - 1; h++)
-                                        if (h < left) mma_step<true>(d, a + h * kStepCols, bd + h * N2, idesc, tmem + kScaleCol);
-                                }
-                                if (tile == 1) tc_commit(&B->exp_empty[as.i]);
-                                bd += kUnitSteps * N2;
-                                left -= kUnitSteps;
-                                as.next(P.ring);
-                            }
-                            tc_commit(&B->d_full[ds.i]);
-                            ds.next(P.n_d);
-                        }
-                        continue;
-                    }
-                    Ring d1 = ds;
-                    d1.next(P.n_d);
-                    warp_wait(&B->d_empty[ds.i], ds.ph ^ 1u, B, P.status);
-                    warp_wait(&B->d_empty[d1.i], d1.ph ^ 1u, B, P.status);
-                    const uint32_t t0 = tmem + ds.i * P.d_cols, t1 = tmem + d1.i * P.d_cols;
+                    warp_wait(&B->d_empty[es.i], es.ph ^ 1u, B, P.status);
+                    const uint32_t d = tmem + (ds.i & (P.n_d - 1)) * P.d_cols;
                     tc_fence_after();
-                    mma_step<false>(t0, tmem + kBiasCol, bias, idesc, tmem + kScaleCol);
-                    mma_step<false>(t1, tmem + kBiasCol, bias, idesc, tmem + kScaleCol);
+                    mma_step<false>(d, tmem + kBiasCol, bias, idesc, tmem + kScaleCol);
                     uint64_t bd = b0;
-                    for (uint32_t s = 0; s < steps;) {
+                    for (uint32_t left = steps; left;) {
                         warp_wait(&B->exp_full[as.i], as.ph, B, P.status);
                         tc_fence_after();
-                        uint32_t a = tmem + a_col + as.i * kUnitCols;
-                        const uint32_t end = umin32(steps, s + kUnitSteps);
-                        for (; s < end; s++) {
-                            mma_step<true>(t0, a, bd, idesc, tmem + kScaleCol);
-                            mma_step<true>(t1, a + kStepCols / 2, bd, idesc, tmem + kScaleCol);
-                            bd += N2;
-                            a += kStepCols;
+                        const uint32_t a = tmem + a_col + as.i * kUnitCols + tile * (kStepCols / 2);
+                        if (left >= kUnitSteps) {
+                            mma_unit(d, a, bd, N2, idesc, tmem + kScaleCol, &B->exp_empty[as.i]);
+                            left -= kUnitSteps;
+                        } else {
+#pragma unroll
+                            for (uint32_t h = 0; h < kUnitSteps - 1; h++)
+                                if (h < left) mma_step<true>(d, a + h * kStepCols, bd + h * N2, idesc, tmem + kScaleCol);
+                            tc_commit(&B->exp_empty[as.i]);
+                            left = 0;
                         }
-                        tc_commit(&B->exp_empty[as.i]);
+                        bd += kUnitSteps * N2;
                         as.next(P.ring);
                     }
                     tc_commit(&B->d_full[ds.i]);
-                    tc_commit(&B->d_full[d1.i]);
-                    ds = d1;
-                    ds.next(P.n_d);
+                    ds.next(kDBars), ds.next(kDBars);
+                    es.next(kDBars), es.next(kDBars);
                 }
                 tc_commit(&B->b_empty[bs.i]);
                 bs.next(P.n_b);
@@ -544,10 +536,10 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
             it.next(kItemSlots);
         }
         // the MMAs in flight end before tensor and shared memory are given up
-        tc_commit(&B->fin);
+        tc_commit(&B->fin[tile]);
         __syncwarp();
         const uint64_t t0 = global_ns();
-        while (!mbar_try_wait(&B->fin, 0) && global_ns() - t0 < 100000000ull) {
+        while (!mbar_try_wait(&B->fin[tile], 0) && global_ns() - t0 < 100000000ull) {
         }
     } else if (warp < kEpiWarp) {
         // ---- builders of the coefficient operand
@@ -631,13 +623,11 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
         }
     } else if (warp < kExpWarp) {
         // ---- epilogue: counts -> parities -> bytes -> rows
-        const uint32_t e = (uint32_t)warp & 3u, tile = (uint32_t)(warp - kEpiWarp) >> 2;  // lane quarter
+        const uint32_t e = (uint32_t)warp & 3u, group = (uint32_t)(warp - kEpiWarp) >> 2;  // lane quarter; blocks
         const uint32_t acc = tmem + (e << 21);
-        const uint32_t pos = G::kElem * (32 * e + lane);  // where this lane's column lies in the tile
-        uint8_t* stg = s_stg + tile * (kGroupBytes * 128);
+        uint8_t* stg = s_stg + (uint32_t)(warp - kEpiWarp) * kEpiStage;
         Ring ds;
-        if (tile) ds.next(P.n_d);
-        uint32_t used = 0;  // tiles so far
+        uint32_t turn = 0;  // the groups take alternate blocks
         for (;;) {
             warp_wait(&B->item_full[it.i], it.ph, B, P.status);
             const ItemSlot& I = H.item[it.i];
@@ -645,77 +635,93 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
             const uint32_t len = uni(I.len), blocks = uni(I.blocks), passes = uni(I.passes), per = uni(I.per),
                            n_out = uni(I.n_out);
             const bool into = uni(I.accumulate) != 0;
+            uint8_t* const out = I.out;
+            const uint64_t stride = I.out_stride;
             for (uint32_t pass = 0; pass < passes; pass++) {
-                const uint32_t lo = pass * per, cnt = umin32(per, n_out - lo);
+                const uint32_t cnt = umin32(per, n_out - pass * per);
                 const uint32_t words = columns_of<kGf16>(cnt) / 32;  // of 4 field bytes
+                const uint8_t* to = I.to + pass * per;
                 for (uint32_t b = 0; b < blocks; b++) {
-                    uint32_t w[4];
-                    warp_wait(&B->d_full[ds.i], ds.ph, B, P.status);
-                    tc_fence_after();
-                    const uint32_t d = acc + ds.i * P.d_cols;
+                    const bool mine = turn == group;
+                    turn ^= 1u;
+                    if (!mine) {
+                        ds.next(kDBars), ds.next(kDBars);
+                        continue;
+                    }
+                    uint32_t w[4][2];  // [word][tile]
 #pragma unroll
-                    for (uint32_t q = 0; q < 4; q += 2) {  // two words' loads in flight
-                        if (q >= words) break;
-                        uint32_t z[2][16];
-                        tmem_load_halves(d + 32 * q, z[0]);
-                        if (q + 1 < words) tmem_load_halves(d + 32 * (q + 1), z[1]);
-                        tmem_wait_load(z[0]);
-                        tmem_wait_load(z[1]);
-                        if (q + 2 >= words) {  // the tile has been read
-                            tc_fence_before();
-                            warp_arrive(&B->d_empty[ds.i], lane);
+                    for (uint32_t tile = 0; tile < 2; tile++) {
+                        warp_wait(&B->d_full[ds.i], ds.ph, B, P.status);
+                        tc_fence_after();
+                        const uint32_t d = acc + (ds.i & (P.n_d - 1)) * P.d_cols;
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; q += 2) {  // two words' loads in flight
+                            if (q >= words) break;
+                            uint32_t z[2][16];
+                            tmem_load_halves(d + 32 * q, z[0]);
+                            if (q + 1 < words) tmem_load_halves(d + 32 * (q + 1), z[1]);
+                            tmem_wait_load(z[0]);
+                            tmem_wait_load(z[1]);
+                            if (q + 2 >= words) {  // the tile has been read
+                                tc_fence_before();
+                                warp_arrive(&B->d_empty[ds.i], lane);
+                            }
+                            w[q][tile] = parity_word(z[0]);
+                            w[q + 1][tile] = parity_word(z[1]);
                         }
-                        w[q] = parity_word(z[0]);
-                        w[q + 1] = parity_word(z[1]);
+                        ds.next(kDBars);
                     }
-                    ds.next(P.n_d);
-                    ds.next(P.n_d);
-                    const uint32_t at = b * G::kRow + tile * G::kTile;
-                    const uint32_t n = len > at ? umin32(G::kTile, len - at) : 0u;  // the row's bytes in this tile
+                    const uint32_t at = b * G::kRow + e * G::kSpan;
+                    const uint32_t n = len > at ? umin32(G::kSpan, len - at) : 0u;  // the row's bytes of these columns
                     if (!cnt || !n) continue;
-                    if (used) {  // the group's last stores have read the staging rows
-                        warp_arrive(&B->stg_empty[tile], lane);
-                        warp_wait(&B->stg_empty[tile], (used - 1) & 1u, B, P.status);
-                    }
+                    __syncwarp();  // the last block's stores have read the staging rows
 #pragma unroll
                     for (uint32_t j = 0; j < G::kGroup; j++) {
                         if (j >= cnt) break;
+                        constexpr uint32_t kWordRows = 4 / G::kElem;  // output rows of a word
+                        const uint32_t* v = w[j / kWordRows];
+                        const uint32_t y = j % kWordRows;
                         if (kGf16)
-                            *reinterpret_cast<uint16_t*>(stg + j * G::kTile + pos) = (uint16_t)(w[j / 2] >> (16 * (j & 1u)));
+                            *reinterpret_cast<uint32_t*>(stg + j * G::kSpan + 4 * lane) = __byte_perm(v[0], v[1], y ? 0x7632 : 0x5410);
                         else
-                            stg[j * G::kTile + pos] = (uint8_t)(w[j / 4] >> (8 * (j & 3u)));
+                            *reinterpret_cast<uint16_t*>(stg + j * G::kSpan + 2 * lane) =
+                                (uint16_t)__byte_perm(v[0], v[1], 0x0040 + 0x0011 * y);
                     }
-                    warp_arrive(&B->stg_full[tile], lane);
-                    warp_wait(&B->stg_full[tile], used & 1u, B, P.status);
-                    used++;
-                    uint8_t* out = I.out + at;
-                    const uint32_t stride = I.out_stride;
+                    __syncwarp();
                     if (kAligned) {
-                        constexpr uint32_t kPieces = G::kTile / kPiece;
-                        for (uint32_t x = 32 * e + lane; x < cnt * kPieces; x += 128) {
-                            const uint32_t j = x / kPieces, o = kPiece * (x % kPieces);
-                            if (o >= n) continue;
-                            Piece v = *reinterpret_cast<const Piece*>(stg + j * G::kTile + o);
-                            Piece* p = reinterpret_cast<Piece*>(out + (uint64_t)I.to[lo + j] * stride + o);
+                        constexpr uint32_t kPieces = G::kSpan / kPiece;
+#pragma unroll
+                        for (uint32_t x = 0; x < G::kGroup * kPieces; x += 32) {
+                            const uint32_t j = (x + lane) / kPieces, o = kPiece * ((x + lane) % kPieces);
+                            if (j >= cnt || o >= n) continue;
+                            Piece v = *reinterpret_cast<const Piece*>(stg + j * G::kSpan + o);
+                            Piece* p = reinterpret_cast<Piece*>(out + to[j] * stride + at + o);
                             if (into) xor_into(v, *p);
                             *p = v;
                         }
                     } else {
-                        for (uint32_t j = e; j < cnt; j += 4) {
-                            uint8_t* row = out + (uint64_t)I.to[lo + j] * stride;
-                            const uint8_t* src = stg + j * G::kTile;
-                            // bytes up to the first whole word of the row, words, the rest
-                            const uint32_t head = umin32((uint32_t)(-reinterpret_cast<intptr_t>(row)) & 3u, n);
-                            const uint32_t full = (n - head) / 4, tail = head + 4 * full;
-                            if ((uint32_t)lane < head) row[lane] = into ? row[lane] ^ src[lane] : src[lane];
-                            for (uint32_t x = lane; x < full; x += 32) {
-                                const uint32_t* s = reinterpret_cast<const uint32_t*>(src + 4 * x);
-                                const uint32_t v = head ? __funnelshift_r(s[0], s[1], 8 * head) : s[0];
-                                uint32_t* p = reinterpret_cast<uint32_t*>(row + head + 4 * x);
-                                *p = into ? *p ^ v : v;
-                            }
-                            if ((uint32_t)lane < n - tail)
-                                row[tail + lane] = into ? row[tail + lane] ^ src[tail + lane] : src[tail + lane];
+                        // bytes up to the first whole word of a row, words, the rest
+                        auto put = [&](uint32_t j, uint32_t o) {
+                            uint8_t* p = out + to[j] * stride + at + o;
+                            const uint8_t v = stg[j * G::kSpan + o];
+                            *p = into ? *p ^ v : v;
+                        };
+                        auto head_of = [&](uint32_t j) {
+                            return umin32((uint32_t)(-reinterpret_cast<intptr_t>(out + to[j] * stride + at)) & 3u, n);
+                        };
+                        for (uint32_t j = (uint32_t)lane / 4; j < cnt; j += 8) {
+                            const uint32_t head = head_of(j), tail = head + ((n - head) & ~3u), y = (uint32_t)lane & 3u;
+                            if (y < head) put(j, y);
+                            if (y < n - tail) put(j, tail + y);
+                        }
+                        constexpr uint32_t kWords = G::kSpan / 4;
+                        for (uint32_t x = lane; x < cnt * kWords; x += 32) {
+                            const uint32_t j = x / kWords, head = head_of(j), o = head + 4 * (x % kWords);
+                            if (o + 4 > n) continue;
+                            const uint32_t* s = reinterpret_cast<const uint32_t*>(stg + j * G::kSpan + (o & ~3u));
+                            const uint32_t v = head ? __funnelshift_r(s[0], s[1], 8 * head) : s[0];
+                            uint32_t* p = reinterpret_cast<uint32_t*>(out + to[j] * stride + at + o);
+                            *p = into ? *p ^ v : v;
                         }
                     }
                 }
@@ -723,176 +729,204 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
             warp_arrive(&B->item_empty[it.i], lane);
             it.next(kItemSlots);
         }
+    } else if (warp >= kLoadWarp) {
+        // ---- loaders: rows -> the staging units
+        const uint32_t t = (uint32_t)(warp - kLoadWarp) * 32 + lane;
+        constexpr uint32_t kPieces = G::kRow / kPiece + (kAligned ? 0 : 1);  // of a row
+        constexpr uint32_t kLoads = (kUnitSteps * G::kStepRows * kPieces + 127) / 128;
+        Ring rs;
+        for (;;) {
+            warp_wait(&B->item_full[it.i], it.ph, B, P.status);
+            const ItemSlot& I = H.item[it.i];
+            if (!uni(I.valid) || aborted(B)) break;
+            const uint32_t len = uni(I.len), passes = uni(I.passes), rows = uni(I.steps) * G::kStepRows;
+            const uint32_t end = kAligned ? len : uni(I.rest);
+            const uint64_t stride = I.in_stride;
+            for (uint32_t pass = 0; pass < passes; pass++)
+                for (uint32_t col = 0; col < len; col += G::kRow)
+                    for (uint32_t row0 = 0; row0 < rows; row0 += kUnitSteps * G::kStepRows) {
+                        const uint8_t* base = I.in + col;
+                        const uint32_t left = umin32(kUnitSteps * G::kStepRows, rows - row0);
+                        uint32_t row[kLoads];  // read ahead of the copies
+#pragma unroll
+                        for (uint32_t x = 0; x < kLoads; x++)
+                            row[x] = I.row[row0 + umin32((128 * x + t) / kPieces, kUnitSteps * G::kStepRows - 1)];
+                        warp_wait(&B->raw_empty[rs.i], rs.ph ^ 1u, B, P.status);
+                        uint8_t* stage = s_raw + rs.i * kUnit;
+#pragma unroll
+                        for (uint32_t x = 0; x < kLoads; x++) {
+                            const uint32_t q = (128 * x + t) / kPieces, o = kPiece * ((128 * x + t) % kPieces);
+                            const uint8_t* p = base + row[x] * stride;
+                            uint32_t lead = 0;
+                            if (!kAligned) {
+                                lead = (uint32_t) reinterpret_cast<uintptr_t>(p) & 15u;
+                                if (q < left && o == 0) stage[kLeads + q] = (uint8_t)lead;
+                            }
+                            copy_in<(int)kPiece>(smem_addr(stage) + q * G::kPitch + o, p - lead + o,
+                                                 q < left && col + o < end + lead);
+                        }
+                        copy_arrive(&B->raw_full[rs.i]);
+                        if (!kAligned) warp_arrive(&B->raw_full[rs.i], lane);
+                        rs.next(kStages);
+                    }
+            warp_arrive(&B->item_empty[it.i], lane);
+            it.next(kItemSlots);
+        }
+        copy_wait_all();
     } else {
         // ---- expanders: rows -> the A operand
         const uint32_t e = (uint32_t)warp & 3u, group = (uint32_t)(warp - kExpWarp) >> 2;
-        uint8_t* units = s_raw + (uint32_t)(warp - kExpWarp) * kDepth * kUnit;
-        // a row's staged bytes: this warp's 32 columns of either tile, in 16-byte
-        // pieces around them when unaligned
-        constexpr uint32_t kPieces = G::kSpan / kPiece + (kAligned ? 0 : 1), kHalf = kPiece * kPieces,
-                           kPitch = 2 * kHalf;
-        constexpr uint32_t kLeads = kStage - 16;  // unaligned: where each row starts in its first piece
-        // a walk over this warp's units, every kExpGroups-th one
-        struct Walk {
-            Ring it;
-            uint32_t unit, col, pass;  // col: bytes from the item's first column
-            uint32_t steps, units, len, passes;
-            bool open, copies;
+        constexpr uint32_t kPitch = G::kPitch;
+        // this warp's units, every kExpGroups-th one
+        uint32_t unit = group, col = 0, pass = 0;  // col: bytes from the item's first column
+        uint32_t n_steps, n_units, len, passes;
+        bool open, with_copies;
+        auto open_item = [&]() {  // the ring's next item, if there is one
+            warp_wait(&B->item_full[it.i], it.ph, B, P.status);
+            const ItemSlot& I = H.item[it.i];
+            open = uni(I.valid) && !aborted(B);
+            n_steps = uni(I.steps), n_units = uni(I.units), len = uni(I.len), passes = uni(I.passes);
+            with_copies = uni(I.copies) != 0;
+            col = pass = 0;
         };
-        auto open_item = [&](Walk& W) {  // the ring's next item, if there is one
-            warp_wait(&B->item_full[W.it.i], W.it.ph, B, P.status);
-            const ItemSlot& I = H.item[W.it.i];
-            W.open = uni(I.valid) && !aborted(B);
-            W.steps = uni(I.steps), W.units = uni(I.units), W.len = uni(I.len), W.passes = uni(I.passes);
-            W.copies = uni(I.copies) != 0;
-            W.col = W.pass = 0;
-        };
-        auto settle = [&](Walk& W, bool release) {  // carries the unit into blocks, passes, items
-            while (W.open && W.unit >= W.units) {
-                W.unit -= W.units;
-                W.col += G::kRow;
-                if (W.col < W.len) continue;
-                W.col = 0;
-                if (++W.pass < W.passes) continue;
-                if (release) warp_arrive(&B->item_empty[W.it.i], lane);
-                W.it.next(kItemSlots);
-                open_item(W);
+        auto settle = [&]() {  // carries the unit into blocks, passes, items
+            while (open && unit >= n_units) {
+                unit -= n_units;
+                col += G::kRow;
+                if (col < len) continue;
+                col = 0;
+                if (++pass < passes) continue;
+                warp_arrive(&B->item_empty[it.i], lane);
+                it.next(kItemSlots);
+                open_item();
             }
         };
-        Walk lw, pw;  // the loads' walk, kDepth units ahead of the work's
-        // the unit's rows into staging slot u
-        auto load_next = [&](uint32_t u) {
-            if (lw.open) {
-                const ItemSlot& I = H.item[lw.it.i];
-                const uint32_t first = lw.col + e * G::kSpan;
-                const uint8_t* base = I.in + first;
-                const uint32_t stride = I.in_stride;
+        // operand bytes of a staged step: w[2 * tile + chunk], this lane's columns
+        auto read_step = [&](const uint8_t* stage, const uint8_t* leads, uint32_t (&w)[4]) {
+            uint32_t x[G::kStepRows];  // both columns' elements of each row
 #pragma unroll
-                for (uint32_t h = 0; h < kUnitSteps; h++) {
-                    const uint32_t step = kUnitSteps * lw.unit + h;
-                    if (step >= lw.steps) break;
-                    uint8_t* stage = units + u * kUnit + h * kStage;
-#pragma unroll
-                    for (uint32_t x = 0; x < G::kStepRows * 2 * kPieces; x += 32) {
-                        const uint32_t g = x + lane, q = g / (2 * kPieces), z = g % (2 * kPieces);
-                        if (g >= G::kStepRows * 2 * kPieces) break;
-                        const uint32_t tile = z / kPieces, o = kPiece * (z % kPieces), at = first + tile * G::kTile + o;
-                        const uint8_t* p = base + (uint64_t)I.row[step * G::kStepRows + q] * stride;
-                        bool has = at < lw.len;
-                        if (!kAligned) {
-                            const uint32_t lead = (uint32_t) reinterpret_cast<uintptr_t>(p) & 15u;
-                            has = at < I.rest + lead;
-                            p -= lead;
-                            if (z == 0) stage[kLeads + q] = (uint8_t)lead;
-                        }
-                        copy_in<(int)kPiece>(smem_addr(stage) + q * kPitch + tile * kHalf + o, p + tile * G::kTile + o, has);
-                    }
+            for (uint32_t q = 0; q < G::kStepRows; q++) {
+                const uint32_t lead = kAligned ? 0u : leads[q];
+                const uint8_t* p = stage + q * kPitch + lead + e * G::kSpan + 2 * G::kElem * lane;
+                if (kGf16) {
+                    const uint32_t* a = reinterpret_cast<const uint32_t*>(p - (lead & 3u));
+                    x[q] = kAligned ? a[0] : __funnelshift_r(a[0], a[1], 8 * (lead & 3u));
+                } else {
+                    x[q] = kAligned ? (uint32_t) *reinterpret_cast<const uint16_t*>(p) : p[0] | (uint32_t)p[1] << 8;
                 }
-                lw.unit += kExpGroups;
-                settle(lw, false);
             }
-            copy_commit();
+#pragma unroll
+            for (int z = 0; z < 2; z++) {
+                if (kGf16) {
+                    w[z] = __byte_perm(x[2 * z], x[2 * z + 1], 0x5410);
+                    w[2 + z] = __byte_perm(x[2 * z], x[2 * z + 1], 0x7632);
+                } else {
+                    const int q = (4 * z) % (int)G::kStepRows;
+                    const uint32_t a = __byte_perm(x[q], x[q + 1], 0x5140);
+                    const uint32_t b = __byte_perm(x[(q + 2) % G::kStepRows], x[(q + 3) % G::kStepRows], 0x5140);
+                    w[z] = __byte_perm(a, b, 0x5410);
+                    w[2 + z] = __byte_perm(a, b, 0x7632);
+                }
+            }
+        };
+        auto write_step = [&](uint32_t dst, const uint32_t (&w)[4]) {
+            tmem_store8(dst, spread(w[0]), spread(w[1]));
+            tmem_store8(dst + kStepCols / 2, spread(w[2]), spread(w[3]));
+        };
+        auto next_slot = [](uint32_t& i, uint32_t& ph, uint32_t n) {
+            i += kExpGroups;
+            if (i >= n) i -= n, ph ^= 1u;
         };
         uint32_t slot = group, slot_ph = 0;  // A slot of this warp's next unit
-        auto work = [&](uint32_t u) {
-            const ItemSlot& I = H.item[pw.it.i];
+        uint32_t raw = group, raw_ph = 0;    // and its staged rows
+        open_item();
+        settle();
+        while (open) {
+            const ItemSlot& I = H.item[it.i];
             const uint32_t dst0 = tmem + (e << 21) + a_col + slot * kUnitCols;
-            const bool copies = pw.copies && pw.pass == 0;  // decode's present rows go straight through
-            const uint32_t first = pw.col + e * G::kSpan;
-            warp_wait(&B->exp_empty[slot], slot_ph ^ 1u, B, P.status);
-            tc_fence_after();
+            const bool copies = with_copies && pass == 0;  // decode's present rows go straight through
+            const uint32_t step0 = kUnitSteps * unit, steps = umin32(kUnitSteps, n_steps - step0);
+            const uint8_t *stage0 = s_raw + raw * kUnit, *leads = stage0 + kLeads;
+            constexpr uint32_t kStep = G::kStepRows * kPitch;
+            warp_wait(&B->raw_full[raw], raw_ph, B, P.status);
+            if (steps == kUnitSteps) {  // read before the slot is free
+                uint32_t w[kUnitSteps][4];
 #pragma unroll
-            for (uint32_t h = 0; h < kUnitSteps; h++) {
-                const uint32_t step = kUnitSteps * pw.unit + h;
-                if (step >= pw.steps) break;
-                const uint8_t* stage = units + u * kUnit + h * kStage;
-                uint4 t[2][2];  // [tile][chunk]: the operand words of this lane's columns
+                for (uint32_t h = 0; h < kUnitSteps; h++) read_step(stage0 + h * kStep, leads + h * G::kStepRows, w[h]);
+                warp_wait(&B->exp_empty[slot], slot_ph ^ 1u, B, P.status);
+                tc_fence_after();
 #pragma unroll
-                for (int tile = 0; tile < 2; tile++) {
-                    uint32_t x[G::kStepRows];  // the column's element of each row
-#pragma unroll
-                    for (uint32_t q = 0; q < G::kStepRows; q++) {
-                        const uint32_t lead = kAligned ? 0u : stage[kLeads + q];
-                        const uint8_t* p = stage + q * kPitch + tile * kHalf + lead + G::kElem * lane;
-                        if (!kGf16)
-                            x[q] = *p;
-                        else if (kAligned || !(lead & 1u))
-                            x[q] = *reinterpret_cast<const uint16_t*>(p);
-                        else
-                            x[q] = p[0] | (uint32_t)p[1] << 8;
-                    }
-#pragma unroll
-                    for (int z = 0; z < 2; z++) {
-                        if (kGf16) {
-                            t[tile][z] = spread(__byte_perm(x[2 * z], x[2 * z + 1], 0x5410));
-                        } else {
-                            const int q = (4 * z) % (int)G::kStepRows;
-                            const uint32_t a = __byte_perm(x[q], x[q + 1], 0x0040);
-                            const uint32_t b = __byte_perm(x[(q + 2) % G::kStepRows], x[(q + 3) % G::kStepRows], 0x0040);
-                            t[tile][z] = spread(__byte_perm(a, b, 0x5410));
-                        }
-                    }
+                for (uint32_t h = 0; h < kUnitSteps; h++) write_step(dst0 + h * kStepCols, w[h]);
+            } else {
+                warp_wait(&B->exp_empty[slot], slot_ph ^ 1u, B, P.status);
+                tc_fence_after();
+#pragma unroll 1
+                for (uint32_t h = 0; h < steps; h++) {
+                    uint32_t w[4];
+                    read_step(stage0 + h * kStep, leads + h * G::kStepRows, w);
+                    write_step(dst0 + h * kStepCols, w);
                 }
-                tmem_store8(dst0 + h * kStepCols, t[0][0], t[0][1]);
-                tmem_store8(dst0 + h * kStepCols + kStepCols / 2, t[1][0], t[1][1]);
             }
             tmem_wait_store();
             tc_fence_before();
+            if (copies) __syncwarp();
+            else warp_arrive(&B->raw_empty[raw], lane);
             warp_arrive(&B->exp_full[slot], lane);
-            slot += kExpGroups;
-            if (slot >= P.ring) slot -= P.ring, slot_ph ^= 1u;
-            if (!copies) return;
-            const uint32_t stride = I.out_stride;
-#pragma unroll
-            for (uint32_t h = 0; h < kUnitSteps; h++) {
-                const uint32_t step = kUnitSteps * pw.unit + h;
-                if (step >= pw.steps) break;
-                const uint8_t* stage = units + u * kUnit + h * kStage;
+            next_slot(slot, slot_ph, P.ring);
+            if (copies) {
+                const uint32_t first = col + e * G::kSpan;
+                uint8_t* const out = I.out + first;
+                const uint64_t stride = I.out_stride;
                 // pieces of aligned rows, words of the others
-                constexpr uint32_t kBy = kAligned ? kPiece : 4, kPer = G::kSpan / kBy;
+                constexpr uint32_t kBy = kAligned ? kPiece : 4, kPer = G::kSpan / kBy, kMoves = G::kStepRows * kPer / 32;
+                if constexpr (kAligned) {
+                    uint32_t to[kUnitSteps][kMoves];  // read ahead of the stores
+                    Piece v[kUnitSteps][kMoves];
 #pragma unroll
-                for (uint32_t x = 0; x < G::kStepRows * 2 * kPer; x += 32) {
-                    const uint32_t g = x + lane, q = g / (2 * kPer), z = g % (2 * kPer), tile = z / kPer;
-                    const uint32_t o = kBy * (z % kPer), at = first + tile * G::kTile + o;
-                    const uint32_t to = I.pass[step * G::kStepRows + q];
-                    if (to == kNoPass || at >= pw.len) continue;
-                    uint8_t* p = I.out + (uint64_t)to * stride + at;
-                    const uint8_t* src = stage + q * kPitch + tile * kHalf + o;
-                    if (kAligned) {
-                        *reinterpret_cast<Piece*>(p) = *reinterpret_cast<const Piece*>(src);
-                    } else {
-                        const uint32_t lead = stage[kLeads + q];
-                        const uint32_t* a = reinterpret_cast<const uint32_t*>(src + (lead & ~3u));
-                        const uint32_t v = __funnelshift_r(a[0], a[1], 8 * (lead & 3u));
-                        if ((reinterpret_cast<uintptr_t>(p) & 3u) == 0 && at + 4 <= pw.len) {
-                            *reinterpret_cast<uint32_t*>(p) = v;
-                        } else {
+                    for (uint32_t h = 0; h < kUnitSteps; h++)
 #pragma unroll
-                            for (uint32_t y = 0; y < 4; y++)
-                                if (at + y < pw.len) p[y] = (uint8_t)(v >> (8 * y));
+                        for (uint32_t x = 0; x < kMoves; x++) {
+                            const uint32_t q = (32 * x + lane) / kPer, o = kBy * ((32 * x + lane) % kPer);
+                            to[h][x] = I.pass[(step0 + h) * G::kStepRows + q];
+                            v[h][x] = *reinterpret_cast<const Piece*>(stage0 + h * kStep + q * kPitch + e * G::kSpan + o);
+                        }
+#pragma unroll
+                    for (uint32_t h = 0; h < kUnitSteps; h++)
+#pragma unroll
+                        for (uint32_t x = 0; x < kMoves; x++) {
+                            const uint32_t o = kBy * ((32 * x + lane) % kPer);
+                            if (h < steps && to[h][x] != kNoPass && first + o < len)
+                                *reinterpret_cast<Piece*>(out + to[h][x] * stride + o) = v[h][x];
+                        }
+                } else {
+#pragma unroll 1
+                    for (uint32_t h = 0; h < steps; h++) {
+                        const uint8_t* stage = stage0 + h * kStep + e * G::kSpan;
+#pragma unroll
+                        for (uint32_t x = 0; x < kMoves; x++) {
+                            const uint32_t q = (32 * x + lane) / kPer, o = kBy * ((32 * x + lane) % kPer), at = first + o;
+                            const uint32_t to = I.pass[(step0 + h) * G::kStepRows + q];
+                            if (to == kNoPass || at >= len) continue;
+                            uint8_t* p = out + to * stride + o;
+                            const uint32_t lead = leads[h * G::kStepRows + q];
+                            const uint32_t* a = reinterpret_cast<const uint32_t*>(stage + q * kPitch + o + (lead & ~3u));
+                            const uint32_t v = __funnelshift_r(a[0], a[1], 8 * (lead & 3u));
+                            if ((reinterpret_cast<uintptr_t>(p) & 3u) == 0 && at + 4 <= len) {
+                                *reinterpret_cast<uint32_t*>(p) = v;
+                            } else {
+#pragma unroll
+                                for (uint32_t y = 0; y < 4; y++)
+                                    if (at + y < len) p[y] = (uint8_t)(v >> (8 * y));
+                            }
                         }
                     }
                 }
+                warp_arrive(&B->raw_empty[raw], lane);
             }
-        };
-        lw.unit = pw.unit = group;
-        open_item(lw);
-        settle(lw, false);
-        // the work's walk starts where the loads' did: items before its first
-        // unit are passed over and released
-        open_item(pw);
-        settle(pw, true);
-        for (uint32_t u = 0; u < kDepth; u++) load_next(u);
-        for (uint32_t u = 0; pw.open; u = u + 1 == kDepth ? 0 : u + 1) {
-            copy_wait<kDepth - 1>();
-            __syncwarp();
-            work(u);
-            __syncwarp();
-            load_next(u);
-            pw.unit += kExpGroups;
-            settle(pw, true);
+            next_slot(raw, raw_ph, kStages);
+            unit += kExpGroups;
+            settle();
         }
-        copy_wait<0>();
     }
     __syncwarp();
     tc_fence_before();
@@ -914,7 +948,7 @@ bool mxt_layout(uint32_t max_in, uint32_t max_out, MxtParams* P) {
     P->n_d = P->d_cols > 64 ? 2 : 4;  // one or two blocks' tiles; the rest is the A ring, three units or more
     P->ring = std::min<uint32_t>(kMaxRing, (kBiasCol - P->n_d * P->d_cols) / kUnitCols);
     P->b_bytes = steps_of<kGf16>(max_in) * P->d_cols * 32;
-    const size_t fixed = up(sizeof(Head), 128) + kBiasBytes + 4 * kExpGroups * kDepth * kUnit + 2 * kGroupBytes * 128 + 16;
+    const size_t fixed = up(sizeof(Head), 128) + kBiasBytes + kStages * kUnit + 8 * kEpiStage;
     for (P->n_b = 2; P->n_b >= 1; P->n_b--)
         if (fixed + (size_t)P->n_b * P->b_bytes <= kMxtSmem) return true;
     return false;
