@@ -221,24 +221,46 @@ int row_align(const MxkTask& T) {
 }
 
 // Whether task T of a device-resident batch drains on the tensor cores
-// (mxt_kernels.cu).  Their time follows the input bytes, the XOR networks'
-// inputs times outputs, so the line lies at a product; below 16 or 24 inputs a
-// K = 64 step is mostly padding.  Rows that are not in 16-byte units cost the
-// XOR networks byte accesses, the tensor cores little.  Measured as time of the
-// XOR networks over time of the tensor cores, batches of 160 MB, 4096-byte rows:
-//   GF(256), k x m:  16 x 16  0.86   24 x 12 1.03   32 x 6 1.07   32 x 8 1.15
-//                    64 x 3  1.16    64 x 16 3.1    128 x 16 3.2   32 x 20 (two passes) 1.11
-//   tower:           8 x 4  0.78     16 x 2 1.08    32 x 1 1.29   32 x 8 3.2   64 x 8 4.5
-// and with 1400-byte rows:
-//   GF(256):         16 x 4 0.92     16 x 5 1.06    24 x 2 1.30   32 x 8 2.8   64 x 16 6.8
-//   tower:           8 x 4  0.99     8 x 6 1.22     16 x 1 1.28   32 x 8 3.4
+// (mxt_kernels.cu).  Their time follows the input bytes, in steps of K = 64 (8 or 4
+// input rows, handed over four at a time), the XOR networks' inputs times outputs;
+// rows that are not in 16-byte units cost the XOR networks byte accesses, the
+// tensor cores little, and a decode its present rows on either side.  So the
+// lines lie at a least number of inputs for some number of outputs.  Measured as time
+// of the XOR networks over time of the tensor cores (batches of 160 MB, whole runs),
+// the last k x m on the left of a line and the first on its right:
+//   GF(256), 4096-byte rows:  16 x 12 0.92 | 16 x 16 1.14   18 x 6 0.94 | 18 x 8 1.02   22 x 4 0.80 | 22 x 5 1.09
+//                             36 x 4 0.82 | 36 x 5 1.05     32 x 2 0.93 | 32 x 4 1.10   44 x 3 0.95 | 44 x 4 1.03
+//                             56 x 1 1.00 | 56 x 2 1.16     64 x 16 2.9 to 3.9          18 x 17 (two passes) 0.96
+//   GF(256), 1400-byte rows:  decode 7 x 1 0.98 | 8 x 1 1.10   32 x 8 4.9
+//                             encode 8 x 5 1.01 | 8 x 8 1.38   10 x 4 1.01 | 10 x 5 1.18   14 x 1 0.96 | 16 x 1 1.12
+//   GF(256), 1401-byte rows:  decode 10 x 2 0.93 | 12 x 4 1.16   encode 16 x 2 0.97 | 17 x 1 1.12   12 x 5 0.88 | 12 x 8 1.06
+//   tower, 4096-byte rows:    8 x 3 0.92 | 8 x 4 1.06   12 x 1 0.88 | 12 x 2 1.05   16 x 1 1.11   32 x 8 2.7 to 3.5
+//   tower, 1400-byte rows:    decode 5 x 2 0.98 | 6 x 1 1.16   encode 6 x 2 0.92 | 6 x 4 1.19   8 x 1 0.91 | 8 x 2 1.08
+//   tower, 1402-byte rows:    decode 6 x 2 1.01 | 8 x 1 1.25   encode 8 x 2 0.93 | 8 x 4 1.08   10 x 1 1.05
 bool on_tensor_cores(const scrs_stripe_batch* b, const MxkTask& T, int gf16) {
     if (b->compact_decode || T.n_out == 0 || T.L >> 32 || !mxt_fits(gf16, T.n_in, T.n_out)) return false;
-    const uint32_t product = T.n_in * T.n_out, passes = (T.n_out + (gf16 ? 7 : 15)) / (gf16 ? 8 : 16);
-    if (row_align(T) == 16) return gf16 ? T.n_in >= 16 && product >= 32 : T.n_in >= 24 && product >= 256 * passes;
-    return gf16 ? T.n_in >= 16 || (T.n_in >= 8 && T.n_out >= 6 && passes == 1)
-                : T.n_in >= 24 || (T.n_in >= 16 && T.n_out >= 5);
+    const uint32_t n = T.n_in, out = T.n_out;
+    const bool decode = T.pass_rows != nullptr;
+    const int align = row_align(T);
+    if (gf16) {
+        if (align == 16) return n >= 16 || (n >= 12 && out >= 2) || (n >= 8 && out >= 4);
+        if (align == 8) return n >= (decode ? 6u : 10u) || (n >= 6 && n * out >= 16);
+        return n >= (decode ? 8u : 10u) || (n >= 8 && out >= 4);
+    }
+    if (align == 16) {
+        if (n < 20 && out > 16) return false;  // two passes over few inputs
+        const uint32_t least = n >= 56 ? 2 : n >= 44 || n % 32 == 0 ? 4 : n >= 21 ? 5 : n >= 18 ? 8 : n >= 16 ? 16 : ~0u;
+        return out >= least;
+    }
+    if (align == 8) return n >= (decode ? 8u : 16u) || (n >= 8 && n * out >= 48);
+    return n >= (decode ? 16u : 17u) || (n >= 12 && out >= (decode ? 4u : 8u));
 }
+
+// Whether stripes of a specialised encode (jit.cu) drain on the tensor cores all
+// the same: rows that are not in 16-byte units cost the specialised networks
+// byte accesses too.  20 x 3: 165 us against 155 (1400-byte rows) and 202 (1401);
+// 32 x 2: 195 us against 100 and 133.
+constexpr uint32_t kTensorOverSpecInputs = 24;
 
 // g^i for i < 65535 (tower/cauchy.rs:44-49) on the current device: the x and
 // y coordinates every tower decode plan reads.  Uploaded once per device.
@@ -530,6 +552,8 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
         for (uint64_t s = 0; s < count; s++) {
             const scrs_stripe_desc& d = descs[s];
             if (d.op != SCRS_OP_ENCODE || d.engine == SCRS_ENGINE_TOWER || !jit_eligible(d.k, d.m)) continue;
+            const MxkTask& T = b->tasks[s];
+            if (d.k >= kTensorOverSpecInputs && row_align(T) < 16 && on_tensor_cores(b, T, 0)) continue;
             auto key = std::make_tuple(d.engine, d.k, d.m);
             auto& g = groups[key];
             if (g.empty()) order.push_back(key);

@@ -56,6 +56,17 @@ def test_geometries_and_alignments(gpu, oracle, engine, align):
     _check(torch, gpu, oracle, _specs(engine, TOWER if engine == Engine.TOWER else GF8, LENGTHS[align], rng), rng)
 
 
+@pytest.mark.parametrize("align", [16, 8, 1])
+@pytest.mark.parametrize("engine", [Engine.GOOD_CAUCHY, Engine.TOWER])
+def test_narrow_codes(gpu, oracle, engine, align):
+    """Codes on both sides of the lines between the two drains."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(300 + align + int(engine))
+    codes = ([(5, 3), (6, 3), (8, 2), (8, 4), (10, 1), (12, 2), (16, 1)] if engine == Engine.TOWER else
+             [(7, 4), (8, 6), (12, 4), (12, 8), (16, 16), (17, 1), (18, 8), (21, 5), (32, 4), (44, 4), (56, 2)])
+    _check(torch, gpu, oracle, _specs(engine, codes, LENGTHS[align], rng), rng)
+
+
 @pytest.mark.parametrize("engine,k,m", [(Engine.STANDARD_CAUCHY, 223, 16), (Engine.STANDARD_CAUCHY, 224, 16),
                                         (Engine.TOWER, 111, 8), (Engine.TOWER, 112, 8)])
 def test_largest_input_counts(gpu, oracle, engine, k, m):
