@@ -208,8 +208,11 @@ constexpr size_t kMaxSpecRuns = 4;  // specialised groups per batch (counters 1.
 constexpr size_t kTowerCounter = 1 + kMaxSpecRuns;  // work counter of the tower drain
 constexpr size_t kMxtCounter = kTowerCounter + 1;   // the tensor-core drains': [field][alignment]
 constexpr size_t kRunCounters = kMxtCounter + 4;
-// Most blocks of a tensor-core item: whole rows up to 8 KiB (16 KiB tower).
-constexpr uint32_t kMxtItemBlocks = 32;
+// Most row bytes of a tensor-core item: whole rows up to 8 KiB.  Longer items leave
+// a longer tail, shorter ones rebuild their coefficient operand more often (tower
+// 32 + 8, 64 KiB rows: 16 KiB items 225 us, 8 KiB 218, 4 KiB 231; mixed GF(256)
+// geometries: 8 KiB 3153 us, 4 KiB 3179, 2 KiB 3305).
+constexpr uint32_t kMxtItemBytes = 8192;
 // Fewest blocks per SM that are worth the kernel's set-up (tensor memory,
 // tables, the first operands: several microseconds).
 constexpr uint32_t kMxtMinBlocksPerSm = 8;
@@ -601,7 +604,7 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
             if (c) b->mxt[f][c - 1].lo = next;
             const uint64_t blocks = c ? b->mxt[f][c - 1].blocks : 0;
             const uint32_t chunk = block * (uint32_t)std::max<uint64_t>(
-                                               1, std::min<uint64_t>(kMxtItemBlocks, blocks / (8ull * b->sm_count)));
+                                               1, std::min<uint64_t>(kMxtItemBytes / block, blocks / (8ull * b->sm_count)));
             for (uint64_t t = 0; t < count; t++) {
                 if (in_spec[t] || b->task_gf16[t] != f) continue;
                 if (on[t] && b->mxt[f][on[t] - 1].blocks < (uint64_t)kMxtMinBlocksPerSm * b->sm_count) on[t] = 0;

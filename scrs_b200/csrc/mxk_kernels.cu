@@ -554,6 +554,7 @@ constexpr uint32_t kPlanRowMinR = 4;
 template <int kGf16>
 __global__ void __launch_bounds__(32 * kPlanWarps) cauchy_plan_warp_kernel(const CauchyPlanTask* __restrict__ tasks,
                                                                           uint32_t n_tasks) {
+    pdl_trigger();  // a drain that follows may start: it waits for the plans where it needs them
     __shared__ Gf8Tables tb;
     __shared__ uint32_t scratch[kPlanWarps][4 * kWarpPlanMaxR];
     for (int i = threadIdx.x; i < 512; i += blockDim.x) {

@@ -42,9 +42,9 @@
 // the ALU pipe 54 %, shared memory 56 % and the issue slots 59 % (4900
 // instructions); the rest is latency between the roles.
 // Drains by CUDA events, whole batches with their plan, half encodes and half decodes
-// of random losses: GF(256) 64 + 16, 4096-byte rows 278 us for 872 MB of rows
+// of random losses: GF(256) 64 + 16, 4096-byte rows 275 us for 872 MB of rows
 // (346 with one issuer, loads in the expanders and 128 separate columns a tile); 32 +
-// 8, 1400-byte rows 238 us for 596 MB (389); tower 32 + 8, 64 KiB rows 282 us
+// 8, 1400-byte rows 231 us for 596 MB (389); tower 32 + 8, 64 KiB rows 258 us
 // for 872 MB (319).
 //
 // Choices, with what the alternatives took.  A lane's two columns neighbours instead
@@ -142,6 +142,7 @@ struct MxtParams {
     uint32_t n_b, b_bytes;      // B slots
     uint32_t d_cols, n_d;       // accumulator tiles: columns each, how many
     uint32_t ring;              // A units, after the accumulators
+    uint32_t smem;              // bytes of shared memory
 };
 
 __host__ __device__ constexpr uint32_t up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
@@ -483,6 +484,7 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
             if (!valid) break;
             it.next(kItemSlots);
         }
+        pdl_wait();  // this launch does not end before the one it started beside
     } else if (warp == 1 || warp == kMma1Warp) {
         // ---- MMA issuers, one for each tile of a block
         const uint32_t tile = warp == 1 ? 0u : 1u;
@@ -545,11 +547,16 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
         // ---- builders of the coefficient operand
         const uint32_t first = (uint32_t)(warp - 2) * 32 + lane;
         Ring bs;
+        bool planned = false;
         for (;;) {
             warp_wait(&B->item_full[it.i], it.ph, B, P.status);
             const ItemSlot& I = H.item[it.i];
             if (!uni(I.valid) || aborted(B)) break;
             const uint32_t n_in = I.n_in, ld = I.ld, passes = uni(I.passes);
+            if (!planned && uni(I.copies)) {  // a decode's coefficients: the plans before this launch
+                pdl_wait();
+                planned = true;
+            }
             const uint16_t* coef_rows = I.coef_rows;
             const void* coef = I.coef;
             for (uint32_t pass = 0; pass < passes; pass++) {
@@ -950,7 +957,10 @@ bool mxt_layout(uint32_t max_in, uint32_t max_out, MxtParams* P) {
     P->b_bytes = steps_of<kGf16>(max_in) * P->d_cols * 32;
     const size_t fixed = up(sizeof(Head), 128) + kBiasBytes + kStages * kUnit + 8 * kEpiStage;
     for (P->n_b = 2; P->n_b >= 1; P->n_b--)
-        if (fixed + (size_t)P->n_b * P->b_bytes <= kMxtSmem) return true;
+        if (const size_t bytes = fixed + (size_t)P->n_b * P->b_bytes; bytes <= kMxtSmem) {
+            P->smem = (uint32_t)bytes;
+            return true;
+        }
     return false;
 }
 
@@ -1002,8 +1012,20 @@ cudaError_t launch_mxt(const MxkTask* tasks, const uint32_t* item_task, uint32_t
     P.chunk = chunk;
     if (grid > (int)(item_end - item_lo)) grid = (int)(item_end - item_lo);
     const MxtFn fn = kMxt[gf16 ? 1 : 0][align >= 16 ? 2 : align >= 8 ? 1 : 0];
-    fn<<<grid, kMxtThreads, kMxtSmem, stream>>>(P);
-    return cudaGetLastError();
+    // Launched beside the batch's plans where they come right before it: only a
+    // decode's coefficients wait for them, so set-up and encodes hide the plan kernel
+    // (1024 stripes of 64 + 16, 4096-byte rows: 158 -> 143 us; 48 + 8: 142 -> 130).
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kMxtThreads);
+    cfg.dynamicSmemBytes = P.smem;  // the least, so that plan blocks fit beside it
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, P);
 }
 
 }  // namespace scrs
