@@ -886,7 +886,10 @@ DrainCfg drain_cfg16(const scrs_stripe_batch* b) {
 // The drains of a device-resident run: the specialised groups' kernels, then
 // the generic drain (work counter q + 1 for group q, 0 for the generic one).
 int32_t enqueue_drains(scrs_stripe_batch* b, cudaStream_t st, scrs_error* err, bool run_spec = true,
-                       bool run_generic = true) {
+                       bool run_generic = true, bool beside_plans = false) {
+    // a launch right after the plan kernel may start beside it (launch_mxt)
+    bool after_plans = beside_plans && !b->plans.empty() && !(run_spec && !b->spec.empty()) && b->alu_hi[0] == b->gen_lo &&
+                       b->alu_hi[1] == b->gen_hi;
     for (size_t q = 0; run_spec && q < b->spec.size(); q++) {
         const scrs_stripe_batch::SpecRun& R = b->spec[q];
         SCRS_CUDA(launch_jit(R.jk, b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), R.item_lo, R.item_hi,
@@ -913,8 +916,9 @@ int32_t enqueue_drains(scrs_stripe_batch* b, cudaStream_t st, scrs_error* err, b
         if (M.hi == M.lo) continue;
         SCRS_CUDA(launch_mxt(b->d_tasks.as<MxkTask>(), b->d_item_task.as<uint32_t>(), M.lo, M.hi,
                              b->d_counter.as<uint32_t>() + kMxtCounter + q, b->status.dev, M.max_in, M.max_out, M.chunk,
-                             b->sm_count, st, M.align, q >> 1));
+                             b->sm_count, st, M.align, q >> 1, after_plans));
         b->last_launches++;
+        after_plans = false;
     }
     return SCRS_OK;
 }
@@ -950,8 +954,8 @@ int32_t enqueue_batch(scrs_stripe_batch* b, cudaStream_t st, scrs_error* err) {
     }
     int32_t rp = enqueue_plans(b, st, err);
     if (rp) return rp;
-    if (!fork) return enqueue_drains(b, st, err);
-    int32_t r = enqueue_drains(b, st, err, false, true);
+    if (!fork) return enqueue_drains(b, st, err, true, true, true);
+    int32_t r = enqueue_drains(b, st, err, false, true, true);
     if (r) return r;
     SCRS_CUDA(cudaEventRecord(b->ev_join, b->s_fork));
     SCRS_CUDA(cudaStreamWaitEvent(st, b->ev_join, 0));

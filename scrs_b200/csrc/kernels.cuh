@@ -114,12 +114,13 @@ cudaError_t launch_gf256_mxk(const MxkTask* tasks, const uint32_t* item_task, ui
 // The same drain on the tensor cores (mxt_kernels.cu), for tasks of at most
 // max_in inputs and max_out outputs (mxt_fits).  An item is `chunk` bytes of the
 // rows, a multiple of mxt_block; align (16, 8 or 1): L and every row of every
-// task are multiples of it.
+// task are multiples of it.  after_plans: the plan kernel of these tasks is the last
+// operation on the stream, and the launch may start beside it.
 bool mxt_fits(int gf16, uint32_t max_in, uint32_t max_out);
 uint32_t mxt_block(int gf16);
 cudaError_t launch_mxt(const MxkTask* tasks, const uint32_t* item_task, uint32_t item_lo, uint32_t item_end,
                        uint32_t* work_counter, int32_t* status, uint32_t max_in, uint32_t max_out, uint32_t chunk,
-                       int grid, cudaStream_t stream, int align, int gf16);
+                       int grid, cudaStream_t stream, int align, int gf16, bool after_plans);
 // Its one-time per-device set-up.
 cudaError_t prepare_mxt();
 // One task by value; grid <= 0 means one CTA per row chunk (or the

@@ -997,7 +997,7 @@ cudaError_t prepare_mxt() { return set_mxt_attrs(); }
 
 cudaError_t launch_mxt(const MxkTask* tasks, const uint32_t* item_task, uint32_t item_lo, uint32_t item_end,
                        uint32_t* counter, int32_t* status, uint32_t max_in, uint32_t max_out, uint32_t chunk, int grid,
-                       cudaStream_t stream, int align, int gf16) {
+                       cudaStream_t stream, int align, int gf16, bool after_plans) {
     if (item_end <= item_lo) return cudaSuccess;
     MxtParams P{};
     if (!layout_for(gf16, max_in, max_out, &P) || chunk == 0 || chunk % mxt_block(gf16)) return cudaErrorInvalidValue;
@@ -1012,7 +1012,8 @@ cudaError_t launch_mxt(const MxkTask* tasks, const uint32_t* item_task, uint32_t
     P.chunk = chunk;
     if (grid > (int)(item_end - item_lo)) grid = (int)(item_end - item_lo);
     const MxtFn fn = kMxt[gf16 ? 1 : 0][align >= 16 ? 2 : align >= 8 ? 1 : 0];
-    // Launched beside the batch's plans where they come right before it: only a
+    // Launched beside the batch's plans where they come right before it (after_plans;
+    // whatever else came before has then ended, and is visible): only a
     // decode's coefficients wait for them, so set-up and encodes hide the plan kernel
     // (1024 stripes of 64 + 16, 4096-byte rows: 158 -> 143 us; 48 + 8: 142 -> 130).
     cudaLaunchAttribute attr[1];
@@ -1024,7 +1025,7 @@ cudaError_t launch_mxt(const MxkTask* tasks, const uint32_t* item_task, uint32_t
     cfg.dynamicSmemBytes = P.smem;  // the least, so that plan blocks fit beside it
     cfg.stream = stream;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = after_plans ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, fn, P);
 }
 
