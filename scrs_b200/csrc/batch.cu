@@ -125,7 +125,8 @@ struct scrs_stripe_batch {
     struct MxtRun {
         uint32_t lo = 0, hi = 0, max_in = 1, max_out = 1, chunk = 0;
         int align = 16;
-        uint64_t blocks = 0;
+        uint64_t blocks = 0, stripes = 0;
+        uint64_t products = 0;  // blocks times the input and output field bytes of a column
     } mxt[2][2];
     uint32_t alu_hi[2] = {0, 0};  // end of each field's multiply-XOR items
     int shape16 = kShapeAny;
@@ -216,6 +217,11 @@ constexpr uint32_t kMxtItemBytes = 8192;
 // Fewest blocks per SM that are worth the kernel's set-up (tensor memory,
 // tables, the first operands: several microseconds).
 constexpr uint32_t kMxtMinBlocksPerSm = 8;
+// Beside other drains of the batch the launch comes on top of theirs (a small one
+// takes 20 to 30 us alone), and it has to save that much: fewest products per SM.
+// Mixed geometries with 1700 lost (260 stripes of k <= 22, m <= 9: 85 -> 105 us), with
+// 14300 gained (624 stripes of k <= 44, m <= 7: 235 -> 219).
+constexpr uint64_t kMxtMinProductsPerSm = 8000;
 
 // Largest of 16, 8 and 1 that every row of T is aligned to.
 int row_align(const MxkTask& T) {
@@ -595,10 +601,18 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
             const int align = row_align(b->tasks[t]);
             on[t] = align == 16 ? 1 : 2;
             scrs_stripe_batch::MxtRun& M = b->mxt[f][on[t] - 1];
-            M.blocks += (b->tasks[t].L + block - 1) / block;
+            const uint64_t blocks = (b->tasks[t].L + block - 1) / block;
+            M.blocks += blocks, M.stripes++;
+            M.products += blocks * b->tasks[t].n_in * b->tasks[t].n_out * (f ? 4 : 1);
             M.max_in = std::max(M.max_in, b->tasks[t].n_in);
             M.max_out = std::max(M.max_out, b->tasks[t].n_out);
             M.align = std::min(M.align, align);
+        }
+        bool worth[2];
+        for (int c = 0; c < 2; c++) {
+            const scrs_stripe_batch::MxtRun& M = b->mxt[f][c];
+            worth[c] = M.blocks >= (uint64_t)kMxtMinBlocksPerSm * b->sm_count &&
+                       (M.stripes == count || M.products >= kMxtMinProductsPerSm * b->sm_count);
         }
         for (int c = 0; c < 3; c++) {
             if (c) b->mxt[f][c - 1].lo = next;
@@ -607,7 +621,7 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
                                                1, std::min<uint64_t>(kMxtItemBytes / block, blocks / (8ull * b->sm_count)));
             for (uint64_t t = 0; t < count; t++) {
                 if (in_spec[t] || b->task_gf16[t] != f) continue;
-                if (on[t] && b->mxt[f][on[t] - 1].blocks < (uint64_t)kMxtMinBlocksPerSm * b->sm_count) on[t] = 0;
+                if (on[t] && !worth[on[t] - 1]) on[t] = 0;
                 if (on[t] != c) continue;
                 MxkTask& T = b->tasks[t];
                 uint32_t& mx = f ? max_in16 : max_in;
