@@ -549,7 +549,6 @@ __global__ void __launch_bounds__(256) cauchy_plan_single(const CauchyPlanTask P
 // scratch.
 constexpr uint32_t kWarpPlanMaxR = 64;
 constexpr int kPlanWarps = 8;
-constexpr uint32_t kPlanRowMinR = 4;
 
 template <int kGf16>
 __global__ void __launch_bounds__(32 * kPlanWarps) cauchy_plan_warp_kernel(const CauchyPlanTask* __restrict__ tasks,
@@ -600,11 +599,13 @@ __global__ void __launch_bounds__(32 * kPlanWarps) cauchy_plan_warp_kernel(const
                 reinterpret_cast<uint8_t*>(P.coef)[(size_t)a * ld + b] = (uint8_t)val;
         }
         // A present column's factor prod_h(z+col_h) / prod_l(z+row_l) takes 2r
-        // products and serves its r entries: with more than a few entries a lane
-        // computes it once and walks the row (k = 64, r = 13: the plans of 1024
-        // decodes 69 -> 22 us; tower k = 32, r = 8: 43 -> 24 us); below that a
-        // lane per entry keeps more lanes busy than the factor costs.
-        for (uint32_t z = lane; r > kPlanRowMinR && z < P.p; z += 32) {
+        // products and serves its r entries.  A lane per row computes it once and
+        // walks the row, 5 r products; a lane per entry repeats it, 2 r + 4 products
+        // for each 32 entries, with more lanes busy.  The shorter chain is taken
+        // (k = 64, r = 13, by rows: the plans of 1024 decodes 69 -> 22 us; tower
+        // k = 32, r = 8: 43 -> 24 us; k = 10 stays by entries).
+        const bool by_row = (P.p * r + 31) / 32 * (2 * r + 4) > (P.p + 31) / 32 * 5 * r;
+        for (uint32_t z = lane; by_row && z < P.p; z += 32) {
             const uint32_t zv = x_var<kGf16>(P, tb, P.present[z]);
             uint32_t rp = 1, cp = 1;
             for (uint32_t h = 0; h < r; h++) {
@@ -621,7 +622,7 @@ __global__ void __launch_bounds__(32 * kPlanWarps) cauchy_plan_warp_kernel(const
                     reinterpret_cast<uint8_t*>(P.coef)[at] = (uint8_t)val;
             }
         }
-        for (uint32_t x = lane; r <= kPlanRowMinR && x < P.p * r; x += 32) {
+        for (uint32_t x = lane; !by_row && x < P.p * r; x += 32) {
             const uint32_t z = x / r, b = x - z * r;  // present row z, output b
             const uint32_t zv = x_var<kGf16>(P, tb, P.present[z]);
             uint32_t rp = 1, cp = 1;
