@@ -551,7 +551,7 @@ def extra_mixed(torch, api, cpu=None):
            "speedup": round(t_plain / t_graph, 2),
            "persistent_ms": round(t_graph, 3), "plain_ms": round(t_plain, 3),
            "persistent_hbm_frac": round(algo / t_graph / 1e6 / peaks()[0], 3),
-           "roofline": roofline_of(algo, t_graph, "plan launch + persistent drain (mxk_kernel), graph replay"),
+           "roofline": roofline_of(algo, t_graph, "plan launch + persistent drains (mxk_kernel, mxt_kernel), graph replay"),
            "autotune": {"default": {"seg_rows": default.seg_rows, "ctas_per_sm": default.ctas_per_sm,
                                     "persistent_ms": round(t_default, 3)},
                         "chosen": {"seg_rows": tuned.seg_rows, "ctas_per_sm": tuned.ctas_per_sm,
@@ -959,7 +959,7 @@ def tower_batched(torch, api, k, m, Lt, rep0, data0, n=128, seed=SEED + 22):
     goodput = 2 * n * k * Lt
     algo = n * (k + m) * Lt + n * 2 * k * Lt
     return {"workload": f"{n} tower encodes + {n} tower decodes (k={k} m={m} L={Lt}, 8 data symbols erased) in one "
-                        "stripe batch: plan launch + persistent drain (mxk_kernel<1>), CUDA graph",
+                        "stripe batch: plan launch + persistent drain (mxt_kernel<1>), CUDA graph",
             "GBps": round(goodput / t / 1e6, 1), "ms": round(t, 3), "launches": b.last_launches,
             "roofline": roofline_of(algo, t, "tower plan + persistent tower drain"), "bit_exact": ok}
 
@@ -1090,7 +1090,7 @@ def extra_sweep(torch, api, cpu=None, ks=(10, 32, 64), ms=(4, 8, 16), Ls=4096, i
         enc_bytes, dec_bytes = n * (k + m) * Ls, n * 2 * k * Ls
         cells.append({"k": k, "m": m, "stripes": n,
                       "encode_ms": round(t_enc, 4), "encode_frac": round(enc_bytes / t_enc / 1e6 / peak, 3),
-                      "encode_kernel": "scrs_spec_drain" if spec else "mxk_kernel<0>",
+                      "encode_kernel": "scrs_spec_drain" if spec else "mxk_kernel<0> or mxt_kernel<0>",
                       "decode_ms": round(t_dec, 4), "decode_frac": round(dec_bytes / t_dec / 1e6 / peak, 3),
                       "decode_plan_ms": round(plan, 4),
                       "mean_erased": round(float((recv >= k).sum()) / n, 2)})

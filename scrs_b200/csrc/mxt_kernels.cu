@@ -38,8 +38,8 @@
 // overlap.
 //
 // What bounds it: no pipe alone.  At 64 inputs and 16 outputs a block takes about
-// 1900 cycles, of which the tensor pipe works 52 % (1150 are the least for 18 MMAs),
-// the ALU pipe 54 %, shared memory 56 % and the issue slots 59 % (4900
+// 2000 cycles, of which the tensor pipe works 55 % (1150 are the least for 18 MMAs),
+// the ALU pipe 59 %, shared memory 56 % and the issue slots 61 % (4900
 // instructions); the rest is latency between the roles.
 // Drains by CUDA events, whole batches with their plan, half encodes and half decodes
 // of random losses: GF(256) 64 + 16, 4096-byte rows 275 us for 872 MB of rows
