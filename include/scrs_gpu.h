@@ -505,6 +505,8 @@ SCRS_API int32_t scrs_jit_prepare(int32_t engine, uint32_t k, uint32_t m, int32_
 SCRS_API int32_t scrs_stripe_batch_set_jit(scrs_stripe_batch* batch, int32_t enable, scrs_error* err);
 /* Stripes of the current descriptors that run through specialised kernels. */
 SCRS_API uint64_t scrs_stripe_batch_jit_stripes(const scrs_stripe_batch* batch);
+/* Stripes of the current descriptors that drain on the tensor cores. */
+SCRS_API uint64_t scrs_stripe_batch_tensor_stripes(const scrs_stripe_batch* batch);
 
 /* The table (for saving and loading it): entries 0..size-1, set, clear. */
 SCRS_API uint64_t scrs_tune_table_size(void);

@@ -255,6 +255,7 @@ extern "C" {
     pub fn scrs_jit_prepare(engine: i32, k: u32, m: u32, load: i32, cubin_bytes: *mut u64, err: *mut scrs_error) -> i32;
     pub fn scrs_stripe_batch_set_jit(batch: *mut scrs_stripe_batch, enable: i32, err: *mut scrs_error) -> i32;
     pub fn scrs_stripe_batch_jit_stripes(batch: *const scrs_stripe_batch) -> u64;
+    pub fn scrs_stripe_batch_tensor_stripes(batch: *const scrs_stripe_batch) -> u64;
     pub fn scrs_tune_table_size() -> u64;
     pub fn scrs_tune_table_entry(i: u64, key: *mut scrs_tune_key, params: *mut scrs_tune_params, err: *mut scrs_error) -> i32;
     pub fn scrs_tune_table_set(key: *const scrs_tune_key, params: *const scrs_tune_params, err: *mut scrs_error) -> i32;

@@ -77,6 +77,8 @@ def _bind(lib: Library):
     L.scrs_stripe_batch_set_jit.argtypes = [C.c_void_p, C.c_int32, C.POINTER(_Error)]
     L.scrs_stripe_batch_jit_stripes.restype = C.c_uint64
     L.scrs_stripe_batch_jit_stripes.argtypes = [C.c_void_p]
+    L.scrs_stripe_batch_tensor_stripes.restype = C.c_uint64
+    L.scrs_stripe_batch_tensor_stripes.argtypes = [C.c_void_p]
     L.scrs_jit_prepare.restype = C.c_int32
     L.scrs_jit_prepare.argtypes = [C.c_int32, C.c_uint32, C.c_uint32, C.c_int32, C.POINTER(C.c_uint64),
                                    C.POINTER(_Error)]
@@ -172,6 +174,11 @@ class StripeBatch:
     def jit_stripes(self) -> int:
         """Stripes of the current descriptors that run through specialised kernels."""
         return int(self._lib.lib.scrs_stripe_batch_jit_stripes(self._ptr))
+
+    @property
+    def tensor_stripes(self) -> int:
+        """Stripes of the current descriptors that drain on the tensor cores."""
+        return int(self._lib.lib.scrs_stripe_batch_tensor_stripes(self._ptr))
 
     def run_plain(self, stream=None):
         err = _Error()

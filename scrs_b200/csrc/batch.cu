@@ -1326,3 +1326,11 @@ extern "C" uint64_t scrs_stripe_batch_jit_stripes(const scrs_stripe_batch* b) {
         for (auto& R : b->spec) n += R.stripes;
     return n;
 }
+
+extern "C" uint64_t scrs_stripe_batch_tensor_stripes(const scrs_stripe_batch* b) {
+    uint64_t n = 0;
+    if (b)
+        for (auto& field : b->mxt)
+            for (auto& M : field) n += M.hi > M.lo ? M.stripes : 0;
+    return n;
+}
