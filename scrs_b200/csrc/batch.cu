@@ -617,8 +617,8 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
         for (int c = 0; c < 3; c++) {
             if (c) b->mxt[f][c - 1].lo = next;
             const uint64_t blocks = c ? b->mxt[f][c - 1].blocks : 0;
-            const uint32_t chunk = block * (uint32_t)std::max<uint64_t>(
-                                               1, std::min<uint64_t>(kMxtItemBytes / block, blocks / (8ull * b->sm_count)));
+            const uint32_t chunk = std::max<uint32_t>(
+                chunk_bytes(f), block * (uint32_t)std::min<uint64_t>(kMxtItemBytes / block, blocks / (8ull * b->sm_count)));
             for (uint64_t t = 0; t < count; t++) {
                 if (in_spec[t] || b->task_gf16[t] != f) continue;
                 if (on[t] && !worth[on[t] - 1]) on[t] = 0;
