@@ -269,7 +269,11 @@ __device__ bool process_item(const MxkTask& T, uint32_t chunk, uint8_t* buf, uin
 }
 
 // Persistent drain: items are claimed from work_counter (or strided by grid
-// when it is nullptr) one ahead of use, so the claim's latency is hidden.
+// when it is nullptr) one ahead of use, so the claim's latency is hidden.  A
+// CTA's first item is its own: were it claimed too, the CTAs that start first
+// would take two before the last have one, and a grid with an item for each
+// CTA would run as long as two (125 decodes of 56 + 2, 4096-byte rows: 80 us
+// or 51, by the order of the claims).
 // Warp 0 loads the current item's descriptor and issues its first stage's
 // copies before the CTA meets at the barrier.
 // Aligned shapes fit 9 CTAs per SM without spilling (2 % faster on cfg1
@@ -284,7 +288,8 @@ __global__ void __launch_bounds__(kThreads, (kShape & kShapeAligned) ? 9 : 8) mx
     const int tid = threadIdx.x;
     uint32_t claims = 0;
     auto claim = [&]() -> uint32_t {
-        const uint32_t v = item_lo + (work_counter ? atomicAdd(work_counter, 1u) : blockIdx.x + claims * gridDim.x);
+        const uint32_t v = item_lo + (work_counter && claims ? gridDim.x + atomicAdd(work_counter, 1u)
+                                                             : blockIdx.x + claims * gridDim.x);
         claims++;
         return v;
     };
