@@ -126,7 +126,7 @@ struct scrs_stripe_batch {
         uint32_t lo = 0, hi = 0, max_in = 1, max_out = 1, chunk = 0;
         int align = 16;
         uint64_t blocks = 0, stripes = 0;
-        uint64_t products = 0;  // blocks times the input and output field bytes of a column
+        double saving[2] = {0, 0};  // SM us saved: each stripe at its alignment, all at 1
     } mxt[2][2];
     uint32_t alu_hi[2] = {0, 0};  // end of each field's multiply-XOR items
     int shape16 = kShapeAny;
@@ -212,16 +212,22 @@ constexpr size_t kRunCounters = kMxtCounter + 4;
 // Most row bytes of a tensor-core item: whole rows up to 8 KiB.  Longer items leave
 // a longer tail, shorter ones rebuild their coefficient operand more often (tower
 // 32 + 8, 64 KiB rows: 16 KiB items 225 us, 8 KiB 218, 4 KiB 231; mixed GF(256)
-// geometries: 8 KiB 3153 us, 4 KiB 3179, 2 KiB 3305).
+// geometries: 8 KiB 3153 us, 4 KiB 3179, 2 KiB 3305).  Batches too small for eight
+// such items per SM take shorter ones, but no less than the chunk that the set counts
+// against the batch's capacity (2 KiB): an item costs 2 us of an SM however short it is
+// (21 + 5, 4096-byte rows, 100 encodes: 32.8 us in items of 256 bytes, 20.5 so).
 constexpr uint32_t kMxtItemBytes = 8192;
 // Fewest blocks per SM that are worth the kernel's set-up (tensor memory,
 // tables, the first operands: several microseconds).
 constexpr uint32_t kMxtMinBlocksPerSm = 8;
-// Beside other drains of the batch the launch comes on top of theirs (a small one
-// takes 20 to 30 us alone), and it has to save that much: fewest products per SM.
-// Mixed geometries with 1700 lost (260 stripes of k <= 22, m <= 9: 85 -> 105 us), with
-// 14300 gained (624 stripes of k <= 44, m <= 7: 235 -> 219).
-constexpr uint64_t kMxtMinProductsPerSm = 8000;
+// Beside other drains of the batch the launch comes on top of theirs and leaves them
+// fewer stripes for the same set-up and tail: microseconds that it has to save.  The
+// XOR networks' launches of unaligned rows have the longer tail.  Least that
+// left no batch slower than without the launch (of 300 mixed-loss ones; 20 for all
+// gave up to 25 % of the tower's gain away, 30 more).  44 + 4, 4096-byte rows, 930
+// decodes: 118 us on the XOR networks, 149 split; 400 of 32 + 8, 1400-byte rows, beside
+// narrow ones are worth theirs.
+constexpr double mxt_beside_us(int align) { return align == 16 ? 8 : 20; }
 
 // Largest of 16, 8 and 1 that every row of T is aligned to.
 int row_align(const MxkTask& T) {
@@ -229,14 +235,59 @@ int row_align(const MxkTask& T) {
     return low % 16 == 0 ? 16 : low % 8 == 0 ? 8 : 1;
 }
 
+// Microseconds of an SM that a stripe of n inputs and m outputs takes less on the tensor
+// cores than on the XOR networks,
+//   n (pairs m + quads ceil(m / 4) + rows + kib L / 1024) + base a pass:
+// in each block of a row that has some, in all for a short row, which costs the XOR
+// networks a whole chunk and the tensor cores 2 us (encode) to 3 us (decode) whatever it
+// holds.  Fitted to drains timed on both sides: 3100 batches of rows of 100 to 1024
+// bytes (16-byte units: up to 2048), and, for the blocks, the difference between
+// batches of 480 and 160 MB of 1100 codes (what a launch costs apart from its
+// stripes is in mxt_beside_us).  Near zero the fit is within 0.2 us a short row
+// and 0.01 to 0.1 us a block.  [field][16, 8 or 1-byte alignment][encode, decode]
+struct Saving {
+    float pairs, quads, rows, kib, base;
+};
+constexpr Saving kShortRowSaving[2][3][2] = {
+    {{{0.0111f, 0.0260f, 0.0655f, -0.0143f, -1.902f}, {0.0124f, 0.0087f, 0.0942f, -0.0065f, -2.371f}},
+     {{0.0146f, 0.0394f, 0.0319f, 0.1117f, -1.836f}, {0.0163f, 0.0214f, 0.0583f, 0.2073f, -2.253f}},
+     {{0.0117f, 0.0296f, 0.0778f, -0.0008f, -1.663f}, {0.0159f, 0.0209f, 0.1005f, 0.0625f, -2.095f}}},
+    {{{0.0354f, 0.0398f, 0.0576f, -0.0157f, -1.707f}, {0.0299f, 0.0636f, 0.0575f, -0.0122f, -2.246f}},
+     {{0.0359f, 0.0630f, 0.0167f, 0.0396f, -1.438f}, {0.0305f, 0.0405f, 0.0400f, 0.1425f, -1.849f}},
+     {{0.0367f, 0.0227f, 0.0786f, 0.0170f, -1.638f}, {0.0327f, 0.0235f, 0.1073f, 0.0581f, -2.008f}}}};
+constexpr Saving kBlockSaving[2][3][2] = {
+    {{{0.0009f, 0.0039f, -0.0038f, 0, -0.190f}, {0.0007f, 0.0043f, -0.0030f, 0, -0.171f}},
+     {{0.0045f, 0.0079f, 0.0171f, 0, -0.397f}, {0.0035f, -0.0012f, 0.0662f, 0, -0.476f}},
+     {{0.0025f, -0.0002f, 0.0367f, 0, -0.574f}, {0.0030f, -0.0058f, 0.0444f, 0, -0.380f}}},
+    {{{0.0088f, -0.0023f, 0.0203f, 0, -0.416f}, {0.0078f, 0.0028f, 0.0185f, 0, -0.430f}},
+     {{0.0117f, 0.0254f, 0.0275f, 0, -0.480f}, {0.0064f, 0.0042f, 0.1341f, 0, -0.761f}},
+     {{0.0071f, 0.0060f, 0.0552f, 0, -0.534f}, {0.0045f, -0.0212f, 0.1397f, 0, -0.577f}}}};
+// A short row that costs up to this much more (within the fit's error) goes with the
+// others: stripes that stay behind need a launch of their own.
+constexpr double kShortRowSlackUs = 0.04;
+bool short_row(const MxkTask& T, int gf16, int align) {
+    return align == 16 ? T.L <= 4ull * mxt_block(gf16) : T.L < 1024;
+}
+double tensor_saving_us(const MxkTask& T, int gf16, int align) {
+    const bool is_short = short_row(T, gf16, align);
+    const Saving& S = (is_short ? kShortRowSaving : kBlockSaving)[gf16][align == 16 ? 0 : align == 8 ? 1 : 2]
+                                                                 [T.pass_rows ? 1 : 0];
+    const uint32_t group = gf16 ? 8 : 16, passes = (T.n_out + group - 1) / group;
+    const uint32_t quads = (T.n_out + 3) / 4;
+    const double each =
+        T.n_in * (S.pairs * T.n_out + S.quads * quads + S.rows + S.kib * (double)T.L / 1024) + S.base * passes;
+    return is_short ? each : each * (double)((T.L + mxt_block(gf16) - 1) / mxt_block(gf16));
+}
+
 // Whether task T of a device-resident batch drains on the tensor cores
 // (mxt_kernels.cu).  Their time follows the input bytes, in steps of K = 64 (8 or 4
 // input rows, handed over four at a time), the XOR networks' inputs times outputs;
 // rows that are not in 16-byte units cost the XOR networks byte accesses, the
 // tensor cores little, and a decode its present rows on either side.  So the
-// lines lie at a least number of inputs for some number of outputs.  Measured as time
-// of the XOR networks over time of the tensor cores (batches of 160 MB, whole runs),
-// the last k x m on the left of a line and the first on its right:
+// lines lie at a least number of inputs for some number of outputs, and short rows, of
+// which the tensor cores pay for whole blocks, have to save time by tensor_saving_us.
+// Measured as time of the XOR networks over time of the tensor cores (batches of
+// 160 MB, whole runs), the last k x m on the left of a line and the first on its right:
 //   GF(256), 4096-byte rows:  16 x 12 0.92 | 16 x 16 1.14   18 x 6 0.94 | 18 x 8 1.02   22 x 4 0.80 | 22 x 5 1.09
 //                             36 x 4 0.82 | 36 x 5 1.05     32 x 2 0.93 | 32 x 4 1.10   44 x 3 0.95 | 44 x 4 1.03
 //                             56 x 1 1.00 | 56 x 2 1.16     64 x 16 2.9 to 3.9          18 x 17 (two passes) 0.96
@@ -251,6 +302,7 @@ bool on_tensor_cores(const scrs_stripe_batch* b, const MxkTask& T, int gf16) {
     const uint32_t n = T.n_in, out = T.n_out;
     const bool decode = T.pass_rows != nullptr;
     const int align = row_align(T);
+    if (short_row(T, gf16, align) && tensor_saving_us(T, gf16, align) < -kShortRowSlackUs) return false;
     if (gf16) {
         if (align == 16) return n >= 16 || (n >= 12 && out >= 2) || (n >= 8 && out >= 4);
         if (align == 8) return n >= (decode ? 6u : 10u) || (n >= 6 && n * out >= 16);
@@ -603,7 +655,8 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
             scrs_stripe_batch::MxtRun& M = b->mxt[f][on[t] - 1];
             const uint64_t blocks = (b->tasks[t].L + block - 1) / block;
             M.blocks += blocks, M.stripes++;
-            M.products += blocks * b->tasks[t].n_in * b->tasks[t].n_out * (f ? 4 : 1);
+            M.saving[0] += tensor_saving_us(b->tasks[t], f, align);
+            if (align < 16) M.saving[1] += tensor_saving_us(b->tasks[t], f, 1);
             M.max_in = std::max(M.max_in, b->tasks[t].n_in);
             M.max_out = std::max(M.max_out, b->tasks[t].n_out);
             M.align = std::min(M.align, align);
@@ -612,7 +665,7 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
         for (int c = 0; c < 2; c++) {
             const scrs_stripe_batch::MxtRun& M = b->mxt[f][c];
             worth[c] = M.blocks >= (uint64_t)kMxtMinBlocksPerSm * b->sm_count &&
-                       (M.stripes == count || M.products >= kMxtMinProductsPerSm * b->sm_count);
+                       (M.stripes == count || M.saving[M.align == 1] >= mxt_beside_us(M.align) * b->sm_count);
         }
         for (int c = 0; c < 3; c++) {
             if (c) b->mxt[f][c - 1].lo = next;
