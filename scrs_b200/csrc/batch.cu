@@ -320,7 +320,8 @@ bool on_tensor_cores(const scrs_stripe_batch* b, const MxkTask& T, int gf16) {
 // Whether stripes of a specialised encode (jit.cu) drain on the tensor cores all
 // the same: rows that are not in 16-byte units cost the specialised networks
 // byte accesses too.  20 x 3: 165 us against 155 (1400-byte rows) and 202 (1401);
-// 32 x 2: 195 us against 100 and 133.
+// 32 x 2: 195 us against 100 and 133.  They stay specialised where the tensor cores
+// are not launched.
 constexpr uint32_t kTensorOverSpecInputs = 24;
 
 // g^i for i < 65535 (tower/cauchy.rs:44-49) on the current device: the x and
@@ -604,17 +605,25 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
     }
     // ---- items: specialised GF(256) encode groups, the generic GF(256)
     // drain's tasks, then the tower tasks (each task in stripe order)
-    b->spec.clear();
-    std::vector<char> in_spec(count, 0);
+    std::vector<char> in_spec;
     uint32_t next = 0;
-    if (b->jit) {
+    // the specialised groups, but for stripes that would rather drain on the tensor
+    // cores (tensor_first); whether there were any
+    auto specialise = [&](bool tensor_first) {
+        b->spec.clear();
+        in_spec.assign(count, 0);
+        next = 0;
+        bool passed = false;
         std::map<std::tuple<int, uint32_t, uint32_t>, std::vector<uint32_t>> groups;
         std::vector<std::tuple<int, uint32_t, uint32_t>> order;  // first appearance
-        for (uint64_t s = 0; s < count; s++) {
+        for (uint64_t s = 0; s < count && b->jit; s++) {
             const scrs_stripe_desc& d = descs[s];
             if (d.op != SCRS_OP_ENCODE || d.engine == SCRS_ENGINE_TOWER || !jit_eligible(d.k, d.m)) continue;
             const MxkTask& T = b->tasks[s];
-            if (d.k >= kTensorOverSpecInputs && row_align(T) < 16 && on_tensor_cores(b, T, 0)) continue;
+            if (tensor_first && d.k >= kTensorOverSpecInputs && row_align(T) < 16 && on_tensor_cores(b, T, 0)) {
+                passed = true;
+                continue;
+            }
             auto key = std::make_tuple(d.engine, d.k, d.m);
             auto& g = groups[key];
             if (g.empty()) order.push_back(key);
@@ -638,14 +647,12 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
             }
             b->spec.push_back({jk, lo, next, (uint64_t)g.size()});
         }
-    }
-    b->gen_lo = next;
-    uint32_t max_in = 1, max_in16 = 1;
-    for (int f = 0; f < 2; f++) {
-        // the tensor-core tasks of each alignment; too few blocks stay with the
-        // others
-        std::vector<uint8_t> on(count, 0);  // 1 + alignment class
-        bool all_aligned = true, all_whole = true;  // of the others
+        return passed;
+    };
+    // the tensor-core tasks of field f by alignment class (`on`: 1 + class), and whether
+    // each class is worth its launch; too few blocks stay with the others
+    auto tensor_classes = [&](int f, std::vector<uint8_t>& on, bool (&worth)[2]) {
+        on.assign(count, 0);
         for (int c = 0; c < 2; c++) b->mxt[f][c] = scrs_stripe_batch::MxtRun{};
         const uint32_t block = mxt_block(f);
         for (uint64_t t = 0; t < count; t++) {
@@ -653,20 +660,33 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
             const int align = row_align(b->tasks[t]);
             on[t] = align == 16 ? 1 : 2;
             scrs_stripe_batch::MxtRun& M = b->mxt[f][on[t] - 1];
-            const uint64_t blocks = (b->tasks[t].L + block - 1) / block;
-            M.blocks += blocks, M.stripes++;
+            M.blocks += (b->tasks[t].L + block - 1) / block, M.stripes++;
             M.saving[0] += tensor_saving_us(b->tasks[t], f, align);
             if (align < 16) M.saving[1] += tensor_saving_us(b->tasks[t], f, 1);
             M.max_in = std::max(M.max_in, b->tasks[t].n_in);
             M.max_out = std::max(M.max_out, b->tasks[t].n_out);
             M.align = std::min(M.align, align);
         }
-        bool worth[2];
         for (int c = 0; c < 2; c++) {
             const scrs_stripe_batch::MxtRun& M = b->mxt[f][c];
             worth[c] = M.blocks >= (uint64_t)kMxtMinBlocksPerSm * b->sm_count &&
                        (M.stripes == count || M.saving[M.align == 1] >= mxt_beside_us(M.align) * b->sm_count);
         }
+    };
+    std::vector<uint8_t> on;
+    bool worth[2];
+    const bool passed = specialise(true);
+    tensor_classes(0, on, worth);
+    if (passed && !worth[1]) {  // no tensor-core launch for the stripes passed over
+        specialise(false);
+        tensor_classes(0, on, worth);
+    }
+    b->gen_lo = next;
+    uint32_t max_in = 1, max_in16 = 1;
+    for (int f = 0; f < 2; f++) {
+        if (f) tensor_classes(f, on, worth);
+        const uint32_t block = mxt_block(f);
+        bool all_aligned = true, all_whole = true;  // of the tasks on the XOR networks
         for (int c = 0; c < 3; c++) {
             if (c) b->mxt[f][c - 1].lo = next;
             const uint64_t blocks = c ? b->mxt[f][c - 1].blocks : 0;
