@@ -469,7 +469,8 @@ typedef struct scrs_tune_params {
 /* Key of a descriptor list (host only; no device work). */
 SCRS_API int32_t scrs_tune_key_of(const scrs_stripe_desc* descs, uint64_t count,
                                   scrs_tune_key* key, scrs_error* err);
-/* Key of the batch's current descriptors. */
+/* Key of the batch's current descriptors, without the stripes that drain on the
+ * tensor cores where others remain. */
 SCRS_API int32_t scrs_stripe_batch_tune_key(const scrs_stripe_batch* batch, scrs_tune_key* key,
                                             scrs_error* err);
 /* The seg_rows and ctas_per_sm a run of the batch would use now. */

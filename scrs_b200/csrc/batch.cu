@@ -133,7 +133,7 @@ struct scrs_stripe_batch {
     std::map<std::pair<uint32_t, uint32_t>, std::vector<uint16_t>> tower_coef;  // host tables by (k, m)
     std::vector<uint16_t> l_row_of, l_missing, l_present, l_repairs;  // per-stripe list scratch
     std::vector<uint8_t> l_seen;
-    scrs_tune_key key{};  // geometry key of the current GF(256) descriptors (autotuner table)
+    scrs_tune_key key{};  // geometry key of the stripes of the GF(256) XOR drain (autotuner table)
     // Encode groups of one (engine, k, m) run through a kernel specialised to
     // their matrix (jit.cu): items [item_lo, item_hi) each; the generic drain
     // takes items [gen_lo, gen_hi).
@@ -595,14 +595,6 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
     b->plans.insert(b->plans.end(), plans16.begin(), plans16.end());
     b->max_plan_r = max_r;
     b->max_plan_r16 = max_r16;
-    if (n_tower) {  // the autotuner's key describes the GF(256) stripes (the drain it tunes)
-        std::vector<scrs_stripe_desc> gf8;
-        for (uint64_t s = 0; s < count; s++)
-            if (descs[s].engine != SCRS_ENGINE_TOWER) gf8.push_back(descs[s]);
-        b->key = tune_key_of(gf8.data(), gf8.size());
-    } else {
-        b->key = tune_key_of(descs, count);
-    }
     // ---- items: specialised GF(256) encode groups, the generic GF(256)
     // drain's tasks, then the tower tasks (each task in stripe order)
     std::vector<char> in_spec;
@@ -682,7 +674,7 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
         tensor_classes(0, on, worth);
     }
     b->gen_lo = next;
-    uint32_t max_in = 1, max_in16 = 1;
+    uint32_t max_in = 1, max_in16 = 1;  // of the tasks on the XOR networks
     for (int f = 0; f < 2; f++) {
         if (f) tensor_classes(f, on, worth);
         const uint32_t block = mxt_block(f);
@@ -697,12 +689,13 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
                 if (on[t] && !worth[on[t] - 1]) on[t] = 0;
                 if (on[t] != c) continue;
                 MxkTask& T = b->tasks[t];
-                uint32_t& mx = f ? max_in16 : max_in;
-                mx = std::max(mx, T.n_in);
-                if (c)
+                if (c) {
                     T.n_items = (uint32_t)((T.L + chunk - 1) / chunk);
-                else
+                } else {
+                    uint32_t& mx = f ? max_in16 : max_in;
+                    mx = std::max(mx, T.n_in);
                     all_aligned &= T.aligned != 0, all_whole &= T.L % FieldGeom<0>::kChunk == 0;
+                }
                 T.item_begin = next;
                 next += T.n_items;
             }
@@ -712,7 +705,22 @@ int32_t scrs::stripe_batch_set_impl(scrs_stripe_batch* b, const scrs_stripe_desc
                 b->alu_hi[f] = next;
         }
         (f ? b->shape16 : b->shape) = !all_aligned ? kShapeAny : all_whole ? (kShapeAligned | kShapeWhole) : kShapeAligned;
-        if (f == 0) b->gen_hi = next;
+        if (f) continue;
+        b->gen_hi = next;
+        // The autotuner's key describes the stripes of the drain it tunes, the GF(256) XOR
+        // networks' (those of the specialised groups among them); where every generic
+        // stripe is on the tensor cores, all GF(256) stripes.
+        const bool xor_drain = b->alu_hi[0] > b->gen_lo;
+        const bool split = xor_drain && b->gen_hi > b->alu_hi[0];
+        if (!xor_drain) max_in = std::max({max_in, b->mxt[0][0].max_in, b->mxt[0][1].max_in});
+        if (n_tower || split) {
+            std::vector<scrs_stripe_desc> tuned;
+            for (uint64_t s = 0; s < count; s++)
+                if (descs[s].engine != SCRS_ENGINE_TOWER && !(split && on[s])) tuned.push_back(descs[s]);
+            b->key = tune_key_of(tuned.data(), tuned.size());
+        } else {
+            b->key = tune_key_of(descs, count);
+        }
     }
     b->total_items = next;
     b->max_in = max_in;
