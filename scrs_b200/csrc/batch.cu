@@ -298,7 +298,7 @@ double tensor_saving_us(const MxkTask& T, int gf16, int align) {
 //   tower, 1400-byte rows:    decode 5 x 2 0.98 | 6 x 1 1.16   encode 6 x 2 0.92 | 6 x 4 1.19   8 x 1 0.91 | 8 x 2 1.08
 //   tower, 1402-byte rows:    decode 6 x 2 1.01 | 8 x 1 1.25   encode 8 x 2 0.93 | 8 x 4 1.08   10 x 1 1.05
 bool on_tensor_cores(const scrs_stripe_batch* b, const MxkTask& T, int gf16) {
-    if (b->compact_decode || T.n_out == 0 || T.L >> 32 || !mxt_fits(gf16, T.n_in, T.n_out)) return false;
+    if (b->compact_decode || T.L >> 32 || !mxt_fits(gf16, T.n_in, T.n_out)) return false;
     const uint32_t n = T.n_in, out = T.n_out;
     const bool decode = T.pass_rows != nullptr;
     const int align = row_align(T);

@@ -111,8 +111,9 @@ constexpr int kShapeAny = 0, kShapeAligned = 1, kShapeWhole = 2, kShapeOneSeg = 
 cudaError_t launch_gf256_mxk(const MxkTask* tasks, const uint32_t* item_task, uint32_t item_lo, uint32_t item_end,
                              uint32_t* work_counter, int32_t* status, int seg_rows, int grid, cudaStream_t stream,
                              int shape = kShapeAny, int gf16 = 0);
-// The same drain on the tensor cores (mxt_kernels.cu), for tasks of at most
-// max_in inputs and max_out outputs (mxt_fits).  An item is `chunk` bytes of the
+// The same drain on the tensor cores (mxt_kernels.cu), for tasks of 1 to max_in inputs
+// and 1 to max_out outputs (mxt_fits) that neither accumulate nor number their
+// coefficient rows (accumulate 0, coef_rows null).  An item is `chunk` bytes of the
 // rows, a multiple of mxt_block; align (16, 8 or 1): L and every row of every
 // task are multiples of it.  after_plans: the plan kernel of these tasks is the last
 // operation on the stream, and the launch may start beside it.

@@ -101,12 +101,11 @@ struct ItemSlot {
     const uint8_t* in;         // at the item's first column
     uint8_t* out;
     const void* coef;
-    const uint16_t* coef_rows;
     uint32_t in_stride, out_stride;
     uint32_t len, rest;        // bytes of the item; and to the end of the rows, up to 16 bytes past the item's
     uint32_t n_in, n_out, ld;
     uint32_t steps, units, passes, per, blocks;
-    uint32_t valid, accumulate, copies;
+    uint32_t valid, copies;
     uint8_t row[kMaxRows];     // input row numbers (row[0] past the end, where coefficients are zero)
     uint8_t pass[kMaxRows];    // output row of a verbatim copy, or kNoPass
     uint8_t to[kMaxRows];      // output row numbers
@@ -298,7 +297,7 @@ __host__ __device__ __forceinline__ uint32_t steps_of(uint32_t n_in) {
 // MMA columns of cnt output rows: 32 for every 4 field bytes.
 template <int kGf16>
 __host__ __device__ __forceinline__ uint32_t columns_of(uint32_t cnt) {
-    return cnt ? up(cnt * MxtGeom<kGf16>::kElem, 4) * 8 : 32u;
+    return up(cnt * MxtGeom<kGf16>::kElem, 4) * 8;
 }
 
 // The four operand words of one chunk: w holds four field bytes.
@@ -320,9 +319,6 @@ __device__ __forceinline__ uint32_t parity_word(const uint32_t (&z)[16]) {
     };
     return pick(0xF0F0F0F0u, nibble(y + 4), nibble(y) >> 4);
 }
-
-__device__ __forceinline__ void xor_into(uint4& a, const uint4& b) { a.x ^= b.x, a.y ^= b.y, a.z ^= b.z, a.w ^= b.w; }
-__device__ __forceinline__ void xor_into(uint2& a, const uint2& b) { a.x ^= b.x, a.y ^= b.y; }
 
 // Asynchronous copy of 16 or 8 bytes into shared memory where `on`.
 template <int kBytes>
@@ -460,7 +456,6 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                     I.in = T.in + off;
                     I.out = T.out + off;
                     I.coef = T.coef;
-                    I.coef_rows = T.coef_rows;
                     I.in_stride = (uint32_t)T.in_stride;
                     I.out_stride = (uint32_t)T.out_stride;
                     const uint64_t rest = T.L - off;
@@ -469,10 +464,9 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                     I.n_in = T.n_in, I.n_out = T.n_out, I.ld = T.ld;
                     I.steps = steps;
                     I.units = (steps + kUnitSteps - 1) / kUnitSteps;
-                    I.passes = T.n_out ? (T.n_out + G::kGroup - 1) / G::kGroup : 1u;  // no outputs: copies alone
+                    I.passes = (T.n_out + G::kGroup - 1) / G::kGroup;
                     I.per = (T.n_out + I.passes - 1) / I.passes;
                     I.blocks = (I.len + G::kRow - 1) / G::kRow;
-                    I.accumulate = T.accumulate;
                     I.copies = T.pass_rows != nullptr;
                 }
                 __syncwarp();  // task is rewritten for the next item
@@ -557,7 +551,6 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                 pdl_wait();
                 planned = true;
             }
-            const uint16_t* coef_rows = I.coef_rows;
             const void* coef = I.coef;
             for (uint32_t pass = 0; pass < passes; pass++) {
                 warp_wait(&B->b_empty[bs.i], bs.ph ^ 1u, B, P.status);
@@ -575,7 +568,7 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                     for (uint32_t q = 0; q < G::kChunkRows; q++) {
                         const uint32_t i = c * G::kChunkRows + q;
                         if (i < n_in) {
-                            const size_t at = (size_t)(coef_rows ? coef_rows[i] : i) * ld + lo + j;
+                            const size_t at = (size_t)i * ld + lo + j;
                             if (kGf16)
                                 v |= (uint32_t) reinterpret_cast<const uint16_t*>(coef)[at] << (16 * q);
                             else
@@ -641,7 +634,6 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
             if (!uni(I.valid) || aborted(B)) break;
             const uint32_t len = uni(I.len), blocks = uni(I.blocks), passes = uni(I.passes), per = uni(I.per),
                            n_out = uni(I.n_out);
-            const bool into = uni(I.accumulate) != 0;
             uint8_t* const out = I.out;
             const uint64_t stride = I.out_stride;
             for (uint32_t pass = 0; pass < passes; pass++) {
@@ -680,7 +672,7 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                     }
                     const uint32_t at = b * G::kRow + e * G::kSpan;
                     const uint32_t n = len > at ? umin32(G::kSpan, len - at) : 0u;  // the row's bytes of these columns
-                    if (!cnt || !n) continue;
+                    if (!n) continue;
                     __syncwarp();  // the last block's stores have read the staging rows
 #pragma unroll
                     for (uint32_t j = 0; j < G::kGroup; j++) {
@@ -701,17 +693,13 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                         for (uint32_t x = 0; x < G::kGroup * kPieces; x += 32) {
                             const uint32_t j = (x + lane) / kPieces, o = kPiece * ((x + lane) % kPieces);
                             if (j >= cnt || o >= n) continue;
-                            Piece v = *reinterpret_cast<const Piece*>(stg + j * G::kSpan + o);
-                            Piece* p = reinterpret_cast<Piece*>(out + to[j] * stride + at + o);
-                            if (into) xor_into(v, *p);
-                            *p = v;
+                            *reinterpret_cast<Piece*>(out + to[j] * stride + at + o) =
+                                *reinterpret_cast<const Piece*>(stg + j * G::kSpan + o);
                         }
                     } else {
                         // bytes up to the first whole word of a row, words, the rest
                         auto put = [&](uint32_t j, uint32_t o) {
-                            uint8_t* p = out + to[j] * stride + at + o;
-                            const uint8_t v = stg[j * G::kSpan + o];
-                            *p = into ? *p ^ v : v;
+                            out[to[j] * stride + at + o] = stg[j * G::kSpan + o];
                         };
                         auto head_of = [&](uint32_t j) {
                             return umin32((uint32_t)(-reinterpret_cast<intptr_t>(out + to[j] * stride + at)) & 3u, n);
@@ -727,8 +715,7 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                             if (o + 4 > n) continue;
                             const uint32_t* s = reinterpret_cast<const uint32_t*>(stg + j * G::kSpan + (o & ~3u));
                             const uint32_t v = head ? __funnelshift_r(s[0], s[1], 8 * head) : s[0];
-                            uint32_t* p = reinterpret_cast<uint32_t*>(out + to[j] * stride + at + o);
-                            *p = into ? *p ^ v : v;
+                            *reinterpret_cast<uint32_t*>(out + to[j] * stride + at + o) = v;
                         }
                     }
                 }
@@ -950,8 +937,8 @@ constexpr size_t kMxtSmem = 227 * 1024;
 template <int kGf16>
 bool mxt_layout(uint32_t max_in, uint32_t max_out, MxtParams* P) {
     using G = MxtGeom<kGf16>;
-    if (max_in == 0 || max_in * G::kElem > kMaxBytes || max_out > kMaxRows) return false;
-    P->d_cols = columns_of<kGf16>(std::max<uint32_t>(1, std::min<uint32_t>(max_out, G::kGroup)));
+    if (max_in == 0 || max_in * G::kElem > kMaxBytes || max_out == 0 || max_out > kMaxRows) return false;
+    P->d_cols = columns_of<kGf16>(std::min<uint32_t>(max_out, G::kGroup));
     P->n_d = P->d_cols > 64 ? 2 : 4;  // one or two blocks' tiles; the rest is the A ring, three units or more
     P->ring = std::min<uint32_t>(kMaxRing, (kBiasCol - P->n_d * P->d_cols) / kUnitCols);
     P->b_bytes = steps_of<kGf16>(max_in) * P->d_cols * 32;
