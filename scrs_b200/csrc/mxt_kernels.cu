@@ -688,13 +688,25 @@ __global__ void __launch_bounds__(kMxtThreads, 1) mxt_kernel(const __grid_consta
                     }
                     __syncwarp();
                     if (kAligned) {
-                        constexpr uint32_t kPieces = G::kSpan / kPiece;
+                        constexpr uint32_t kPieces = G::kSpan / kPiece, kMoves = G::kGroup * kPieces / 32;
+                        // Both 16-byte pieces of a lane are read ahead of the stores (tower 32 + 8
+                        // decodes 180 us, 183 one by one), not four of 8 bytes (1400-byte rows 233 and 228).
+                        constexpr uint32_t kAtOnce = kPiece == 16 ? kMoves : 1;
 #pragma unroll
-                        for (uint32_t x = 0; x < G::kGroup * kPieces; x += 32) {
-                            const uint32_t j = (x + lane) / kPieces, o = kPiece * ((x + lane) % kPieces);
-                            if (j >= cnt || o >= n) continue;
-                            *reinterpret_cast<Piece*>(out + to[j] * stride + at + o) =
-                                *reinterpret_cast<const Piece*>(stg + j * G::kSpan + o);
+                        for (uint32_t x0 = 0; x0 < kMoves; x0 += kAtOnce) {
+                            Piece v[kAtOnce];
+                            uint32_t row[kAtOnce];
+#pragma unroll
+                            for (uint32_t x = 0; x < kAtOnce; x++) {
+                                const uint32_t q = 32 * (x0 + x) + lane, j = q / kPieces, o = kPiece * (q % kPieces);
+                                v[x] = *reinterpret_cast<const Piece*>(stg + j * G::kSpan + o);
+                                row[x] = j < cnt ? to[j] : 0;
+                            }
+#pragma unroll
+                            for (uint32_t x = 0; x < kAtOnce; x++) {
+                                const uint32_t q = 32 * (x0 + x) + lane, j = q / kPieces, o = kPiece * (q % kPieces);
+                                if (j < cnt && o < n) *reinterpret_cast<Piece*>(out + row[x] * stride + at + o) = v[x];
+                            }
                         }
                     } else {
                         // bytes up to the first whole word of a row, words, the rest
