@@ -1070,7 +1070,7 @@ def extra_sweep(torch, api, cpu=None, ks=(10, 32, 64), ms=(4, 8, 16), Ls=4096, i
         torch.cuda.synchronize()
         enc = [b.run_timed_drains() for _ in range(5)]
         t_enc = float(np.median([r[1] + r[2] for r in enc]))
-        spec = b.jit_stripes > 0
+        enc_kernel = ("scrs_spec_drain" if b.jit_stripes else "mxt_kernel<0>" if b.tensor_stripes else "mxk_kernel<0>")
         rng = np.random.default_rng(SEED + 200 + k * 17 + m)
         recv = np.argsort(rng.random((n, k + m)), axis=1)[:, :k].astype(np.int64)
         word = torch.cat([data.view(n, k, Ls), reps.view(n, m, Ls)], dim=1)
@@ -1090,7 +1090,7 @@ def extra_sweep(torch, api, cpu=None, ks=(10, 32, 64), ms=(4, 8, 16), Ls=4096, i
         enc_bytes, dec_bytes = n * (k + m) * Ls, n * 2 * k * Ls
         cells.append({"k": k, "m": m, "stripes": n,
                       "encode_ms": round(t_enc, 4), "encode_frac": round(enc_bytes / t_enc / 1e6 / peak, 3),
-                      "encode_kernel": "scrs_spec_drain" if spec else "mxk_kernel<0> or mxt_kernel<0>",
+                      "encode_kernel": enc_kernel,
                       "decode_ms": round(t_dec, 4), "decode_frac": round(dec_bytes / t_dec / 1e6 / peak, 3),
                       "decode_plan_ms": round(plan, 4),
                       "mean_erased": round(float((recv >= k).sum()) / n, 2)})

@@ -38,11 +38,11 @@
 // overlap.
 //
 // What bounds it: no pipe alone.  At 64 inputs and 16 outputs a block takes about
-// 2000 cycles, of which the tensor pipe works 55 % (1150 are the least for 18 MMAs),
-// the ALU pipe 59 %, shared memory 56 % and the issue slots 61 % (4900
+// 2000 cycles, of which the tensor pipe works 56 % (1150 are the least for 18 MMAs),
+// the ALU pipe 59 %, shared memory 57 % and the issue slots 62 % (4850
 // instructions); the rest is latency between the roles.
 // Drains by CUDA events, whole batches with their plan, half encodes and half decodes
-// of random losses: GF(256) 64 + 16, 4096-byte rows 275 us for 872 MB of rows
+// of random losses: GF(256) 64 + 16, 4096-byte rows 276 us for 872 MB of rows
 // (346 with one issuer, loads in the expanders and 128 separate columns a tile); 32 +
 // 8, 1400-byte rows 231 us for 596 MB (389); tower 32 + 8, 64 KiB rows 258 us
 // for 872 MB (319).
